@@ -194,15 +194,23 @@ typedef struct {
 
 /* Box means of every radius from the SAT. */
 satgb_status satgb_box_filter_fwd(const satgb_box_desc* desc, satgb_stream stream);
+/* Box means of every radius straight from the image d_x (n_planes planes of
+ * width x height f32, pitch and plane stride in elements), in one launch that
+ * writes no SAT.  desc->d_sat (with its pitch and plane stride) is a scratch
+ * SAT for radii too large for that kernel's shared memory (above 64, or their
+ * planes narrower than their windows); without one (NULL) such a call returns
+ * SATGB_ERR_NOT_FOUND.  The means may not overlap the image. */
+satgb_status satgb_box_filter_fwd_x(const satgb_box_desc* desc, const void* d_x, int64_t x_pitch,
+                                    int64_t x_plane_stride, satgb_stream stream);
 /* The adjoint of satgb_box_filter_fwd: dL/dSAT from the gradients of all the
  * radii's means (the four-corner scatter, computed as a gather so it is
  * deterministic).  d_sat is overwritten. */
 satgb_status satgb_box_filter_bwd(const satgb_box_desc* desc, satgb_stream stream);
 /* The gradient of the box means with respect to the image the SAT was taken
- * of, dL/dx = reverse SAT of dL/dSAT, in one call and without scratch memory:
- * dL/dSAT is gathered into d_dx, then d_dx is reverse-summed in place (two
- * tile launches and the edge launch of satgb_box_filter_bwd).  desc->d_sat is
- * not used; d_dx (n_planes planes of width x height, pitch and plane stride in
+ * of, in one call and without scratch memory: one launch of window sums of the
+ * means' gradients, or, for radii too large for that kernel's shared memory,
+ * dL/dSAT gathered into d_dx and reverse-summed in place (two tile launches
+ * and the edge launch of satgb_box_filter_bwd).  desc->d_sat is not used; d_dx (n_planes planes of width x height, pitch and plane stride in
  * elements) is written and may not overlap the gradients of the means. */
 satgb_status satgb_box_filter_bwd_x(const satgb_box_desc* desc, void* d_dx, int64_t dx_pitch,
                                     int64_t dx_plane_stride, satgb_stream stream);

@@ -250,6 +250,26 @@ def box_means_from_sat(sat_t: torch.Tensor, radii: Sequence[int], out=None, stre
     return out
 
 
+def box_means(x: torch.Tensor, radii: Sequence[int], out=None, stream=None) -> torch.Tensor:
+    """Clipped box means of every radius of the image x itself: (..., H, W) ->
+    (..., R, H, W), in one launch; radii too large for that launch go through
+    the SAT of x in a scratch tensor."""
+    if out is None:
+        out = torch.empty(x.shape[:-2] + (len(radii),) + x.shape[-2:], dtype=torch.float32, device=x.device)
+    d = _box_desc(x, out, radii)
+    dx, pitch, plane = d.d_sat, d.sat_pitch, d.sat_plane_stride
+    d.d_sat = None
+    L = _lib.load()
+    st = L.satgb_box_filter_fwd_x(ctypes.byref(d), dx, pitch, plane, _stream_handle(stream))
+    if st == _lib.ERR_NOT_FOUND:
+        scratch = torch.empty(x.shape, dtype=torch.float32, device=x.device)
+        s3 = scratch if scratch.dim() >= 3 else scratch.unsqueeze(0)
+        d.d_sat, d.sat_pitch, _, _, _, d.sat_plane_stride = _planes_args(s3)
+        st = L.satgb_box_filter_fwd_x(ctypes.byref(d), dx, pitch, plane, _stream_handle(stream))
+    check(st)
+    return out
+
+
 def box_means_adjoint(grad_boxes: torch.Tensor, radii: Sequence[int], out=None, stream=None) -> torch.Tensor:
     """The adjoint of box_means_from_sat: dL/dSAT (..., H, W) from dL/dmeans
     (..., R, H, W)."""

@@ -22,6 +22,7 @@ GENCODE = "-gencode=arch=compute_103a,code=sm_103a"
 
 SOURCES = [
     "satgb_api.cu",
+    "box_fused.cu",
     "sat_inst_u8.cu",
     "sat_inst_i8.cu",
     "sat_inst_int32.cu",

@@ -20,6 +20,7 @@
 #include <cstdint>
 
 #include "../../include/satgb.h"
+#include "box_args.h"
 
 namespace satgb {
 satgb_status api_fail(satgb_status st, const char* msg);
@@ -27,20 +28,9 @@ satgb_status api_cuda_fail(cudaError_t e, const char* what);
 void api_count_launch();
 }  // namespace satgb
 
-namespace {
+using satgb::BoxArgs;
 
-struct BoxArgs {
-  int64_t w, h, planes;
-  float* sat;
-  int64_t sat_pitch, sat_plane;
-  int nr;
-  int rmax; // the largest radius
-  int r[SATGB_MAX_RADII];
-  float inv_full[SATGB_MAX_RADII]; // 1 / (2r + 1): the reciprocal window length away from the edges
-  float* box[SATGB_MAX_RADII];
-  int64_t box_pitch, box_plane;
-  int idx32; // every in-plane element offset fits in 32 bits: only then the interior paths run (int offsets)
-};
+namespace {
 
 // A block covers 32 columns x 64 rows of one plane: blockDim (32, 8), each
 // thread 8 rows 8 apart, so a warp touches 32 consecutive columns of a row.
@@ -330,13 +320,6 @@ __global__ void __launch_bounds__(kEdgeThreads) box_bwd_edge_kernel(const __grid
 
 satgb_status check_desc_(const satgb_box_desc* d, BoxArgs& a);
 
-satgb_status check_desc(const satgb_box_desc* d, BoxArgs& a) {
-  const satgb_status st = check_desc_(d, a);
-  if (st == SATGB_ERR_MISALIGNED) return satgb::api_fail(st, "box filter: f32 pointer not 4-byte aligned");
-  if (st != SATGB_OK) return satgb::api_fail(st, "box filter: invalid descriptor (sizes, pitches, radii or pointers)");
-  return st;
-}
-
 satgb_status check_desc_(const satgb_box_desc* d, BoxArgs& a) {
   if (!d) return SATGB_ERR_INVALID_ARG;
   if (d->width < 0 || d->height < 0 || d->n_planes < 0) return SATGB_ERR_INVALID_ARG;
@@ -383,9 +366,18 @@ satgb_status check_desc_(const satgb_box_desc* d, BoxArgs& a) {
 
 }  // namespace
 
+namespace satgb {
+satgb_status box_check_desc(const satgb_box_desc* d, BoxArgs& a) {
+  const satgb_status st = check_desc_(d, a);
+  if (st == SATGB_ERR_MISALIGNED) return api_fail(st, "box filter: f32 pointer not 4-byte aligned");
+  if (st != SATGB_OK) return api_fail(st, "box filter: invalid descriptor (sizes, pitches, radii or pointers)");
+  return st;
+}
+}  // namespace satgb
+
 extern "C" satgb_status satgb_box_filter_fwd(const satgb_box_desc* d, satgb_stream stream) {
   BoxArgs a;
-  satgb_status st = check_desc(d, a);
+  satgb_status st = satgb::box_check_desc(d, a);
   if (st != SATGB_OK || d->width == 0 || d->height == 0 || d->n_planes == 0) return st;
   dim3 grid((unsigned)((d->width + kBX - 1) / kBX), (unsigned)((d->height + kBY * kRows - 1) / (kBY * kRows)),
             (unsigned)d->n_planes);
@@ -405,7 +397,7 @@ extern "C" satgb_status satgb_box_filter_fwd(const satgb_box_desc* d, satgb_stre
 
 extern "C" satgb_status satgb_box_filter_bwd(const satgb_box_desc* d, satgb_stream stream) {
   BoxArgs a;
-  satgb_status st = check_desc(d, a);
+  satgb_status st = satgb::box_check_desc(d, a);
   if (st != SATGB_OK || d->width == 0 || d->height == 0 || d->n_planes == 0) return st;
   dim3 grid((unsigned)((d->width + kBX - 1) / kBX), (unsigned)((d->height + kBY * kBRows - 1) / (kBY * kBRows)),
             (unsigned)d->n_planes);

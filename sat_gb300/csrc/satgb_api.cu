@@ -21,6 +21,7 @@
 
 #include "../../include/satgb.h"
 #include "batch_repack.h"
+#include "box_args.h"
 #include "sat_kernel.cuh"
 #include "sat_registry.h"
 
@@ -948,6 +949,40 @@ satgb_status satgb_autotune(satgb_dtype in_t, satgb_dtype out_t, int mode, const
 // ---------------------------------------------------------------------------
 // box-filter backward to the image
 // ---------------------------------------------------------------------------
+satgb_status satgb_box_filter_fwd_x(const satgb_box_desc* desc, const void* d_x, int64_t x_pitch,
+                                    int64_t x_plane_stride, satgb_stream stream) {
+  if (!desc) return fail(SATGB_ERR_INVALID_ARG, "box means: null descriptor");
+  const long long w = desc->width, h = desc->height, planes = desc->n_planes;
+  satgb_box_desc d = *desc;
+  d.d_sat = const_cast<void*>(d_x);
+  d.sat_pitch = x_pitch;
+  d.sat_plane_stride = planes > 1 ? x_plane_stride : 0;
+  satgb::BoxArgs a;
+  satgb_status st = satgb::box_check_desc(&d, a);
+  if (st != SATGB_OK || w == 0 || h == 0 || planes == 0) return st;
+  // no box plane may overlap the image it is computed from
+  const long long xspan = (h - 1) * x_pitch + w + (planes - 1) * d.sat_plane_stride;
+  const long long bspan = (h - 1) * desc->box_pitch + w + (planes - 1) * (planes > 1 ? desc->box_plane_stride : 0);
+  const char* xb = (const char*)d_x;
+  for (int i = 0; i < desc->n_radii; ++i) {
+    const char* bb = (const char*)desc->d_box[i];
+    if (xb < bb + bspan * 4 && bb < xb + xspan * 4)
+      return fail(SATGB_ERR_INVALID_ARG, "box means: the means overlap the image");
+  }
+  bool done = false;
+  st = satgb::box_means_fused(a, (cudaStream_t)stream, &done);
+  if (st != SATGB_OK || done) return st;
+  if (!desc->d_sat)
+    return fail(SATGB_ERR_NOT_FOUND, "box means: these radii need a scratch SAT (descriptor's d_sat)");
+  const long long splane = planes > 1 ? desc->sat_plane_stride : 0;
+  if (desc->sat_pitch < w || (planes > 1 && splane < (h - 1) * desc->sat_pitch + w))
+    return fail(SATGB_ERR_INVALID_ARG, "box means: scratch SAT pitch or plane stride too small");
+  st = sat_single(SATGB_F32, SATGB_F32, SATGB_MODE_PLAIN, SATGB_FORWARD, d_x, x_pitch, desc->d_sat, desc->sat_pitch, w, h,
+                  (cudaStream_t)stream, -1, planes, d.sat_plane_stride, splane);
+  if (st != SATGB_OK) return st;
+  return satgb_box_filter_fwd(desc, stream);
+}
+
 satgb_status satgb_box_filter_bwd_x(const satgb_box_desc* desc, void* d_dx, int64_t dx_pitch,
                                     int64_t dx_plane_stride, satgb_stream stream) {
   if (!desc) return fail(SATGB_ERR_INVALID_ARG, "box filter backward: null descriptor");
@@ -971,12 +1006,18 @@ satgb_status satgb_box_filter_bwd_x(const satgb_box_desc* desc, void* d_dx, int6
         return fail(SATGB_ERR_INVALID_ARG, "box filter backward: the gradient output overlaps the gradients of the means");
     }
   }
-  // dL/dSAT into the output, then its reverse SAT in place
   satgb_box_desc d = *desc;
   d.d_sat = d_dx;
   d.sat_pitch = dx_pitch;
   d.sat_plane_stride = planes > 1 ? dx_plane_stride : 0;
-  satgb_status st = satgb_box_filter_bwd(&d, stream);
+  satgb::BoxArgs a;
+  satgb_status st = satgb::box_check_desc(&d, a);
+  if (st != SATGB_OK) return st;
+  bool done = false;
+  st = satgb::box_grad_fused(a, (cudaStream_t)stream, &done);
+  if (st != SATGB_OK || done) return st;
+  // dL/dSAT into the output, then its reverse SAT in place
+  st = satgb_box_filter_bwd(&d, stream);
   if (st != SATGB_OK) return st;
   return sat_single(SATGB_F32, SATGB_F32, SATGB_MODE_PLAIN, SATGB_REVERSE, d_dx, dx_pitch, d_dx, dx_pitch, w, h,
                     (cudaStream_t)stream, -1, planes, d.sat_plane_stride, d.sat_plane_stride);

@@ -317,3 +317,55 @@ def test_grad_x_pitched_planes(cuda):
     ref = sat_gb300.sat(api.box_means_adjoint(wts.contiguous(), (2, 5)), torch.float32, reverse=True)
     assert float((out - ref).abs().max()) <= 1e-5 * max(1.0, float(ref.abs().max()))
     assert bool(torch.isnan(out_base[..., 90:]).all())  # the row padding is never written
+
+
+def window_error(r, area=True):
+    """Bound of a window sum's rounding error over N(0, 1) inputs in the one-launch
+    kernels, over the smallest clipped area: a column's running sum is updated twice a
+    row for at most 256 rows (|V| <= 6 sqrt(2r + 1)) and enters 2r + 1 times; a prefix
+    over 256 columns of them (|p| <= 96 sqrt(2r + 1)) carries at most 40 roundings."""
+    eps, n = 2.0 ** -24, 2 * r + 1
+    return eps * n ** 0.5 * (256 * 6 * n + 40 * 96) / (r + 1) ** 2
+
+
+@pytest.mark.parametrize("shape,radii", [
+    ((1, 2, 33, 224), (15,)),          # one whole block of 7 column groups
+    ((2, 1, 129, 225), (3, 7, 15)),    # one column past it, one row past a strip, rows unaligned
+    ((1, 1, 70, 448), (3, 7, 15)),     # two whole blocks
+    ((1, 3, 40, 31), (0, 1, 2, 30)),   # narrower than a column group, windows wider than the plane
+    ((1, 1, 300, 260), (11, 31)),      # aligned rows, last group not whole
+    ((1, 1, 1, 500), (5,)), ((1, 1, 500, 1), (5,)), ((1, 1, 1, 1), (2,)),
+    ((1, 2, 150, 300), (0, 15)), ((2, 1, 90, 100), (3, 3, 7)),  # radius 0; a radius twice
+    ((1, 1, 140, 200), (64,)),         # too large for the one-launch kernels
+])
+def test_box_layer_windows(cuda, shape, radii):
+    """Box means straight from the image and their gradient, at the edges of the
+    kernels' blocks, strips and column groups, against float64."""
+    g = torch.Generator(device="cpu").manual_seed(29)
+    x = torch.randn(shape, generator=g).to(cuda).requires_grad_(True)
+    w = torch.randn(shape[:-2] + (len(radii),) + shape[-2:], generator=g).to(cuda)
+    m = AG.box_filter_means(x, radii)
+    m.backward(w)
+    x64 = x.detach().double().requires_grad_(True)
+    m64 = box_means64(x64, radii)
+    m64.backward(w.double())
+    for k, r in enumerate(radii):
+        err = float((m[..., k, :, :].double() - m64[..., k, :, :]).abs().max())
+        assert err <= window_error(r), (r, err)
+    err = float((x.grad.double() - x64.grad).abs().max())
+    assert err <= sum(window_error(r) for r in radii), err
+
+
+def test_box_layer_views_and_offsets(cuda):
+    """Pitched planes and a base that is not 16-byte aligned, and outputs whose row
+    padding stays untouched."""
+    g = torch.Generator(device="cpu").manual_seed(30)
+    base = torch.randn((3, 50, 260), generator=g).to(cuda)
+    for x in (base[..., :256], base[..., 1:250], base[..., 4:260]):
+        h, w = x.shape[-2:]
+        out = torch.full((3, 2, h, w + 4), float("nan"), device=cuda)
+        m = api.box_means(x, (3, 9), out=out[..., :w])
+        ref = box_means64(x, (3, 9))
+        for k, r in enumerate((3, 9)):
+            assert float((m[:, k].double() - ref[:, k]).abs().max()) <= window_error(r)
+        assert bool(torch.isnan(out[..., w:]).all())
