@@ -157,9 +157,7 @@ __global__ void __launch_bounds__(TileShapeRM<TIn, TOut, A, RPW, NWC>::THREADS, 
   const uint32_t tagA = make_tag(epoch, kStateAgg);
   const uint32_t tagI = make_tag(epoch, kStateInc);
 
-  // ---- prologue: the producer fills every stage ---------------------------------
-  bool producing = true;
-  unsigned long long pending = 0;
+  // ---- prologue: barriers; the producer fills the stages while the other roles start ------------
   if (warp == WPROD && lane == 0) {
 #pragma unroll
     for (int s = 0; s < S; ++s) {
@@ -167,6 +165,12 @@ __global__ void __launch_bounds__(TileShapeRM<TIn, TOut, A, RPW, NWC>::THREADS, 
       mbar_init(smem_u32(&s_done[s]), NWC);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+
+  bool producing = true;
+  unsigned long long pending = 0;
+  if (warp == WPROD && lane == 0) {
     for (int s = 0; s < S && producing; ++s) {
       const TilePlan tp = plan_tile<REV, kOrderRows>(P, atomicAdd(&P.ws->ticket, 1ull));
       issue_tile<TIn, TW, TH, SH::IN_BYTES>(P, tp, s, stages + s * STAGE_ELEMS, s_tile, s_img, s_tx, s_ty, s_pl,
@@ -175,7 +179,6 @@ __global__ void __launch_bounds__(TileShapeRM<TIn, TOut, A, RPW, NWC>::THREADS, 
     }
     if (producing) pending = atomicAdd(&P.ws->ticket, 1ull);
   }
-  __syncthreads();
 
   if (warp == WPROD && lane == 0) {
     // ---- producer: each stage is refilled once the output phase has read it -----

@@ -130,11 +130,8 @@ __global__ void __launch_bounds__(TileShapeWS<TIn, TOut, A, RPW, NWC, DIRECT, CT
   const uint32_t tagA = make_tag(epoch, kStateAgg);
   const uint32_t tagI = make_tag(epoch, kStateInc);
 
-  // ---- prologue: the store warp fills every stage -----------------------------
+  // ---- prologue: barriers; the store warp fills the stages while the other roles start --------
   if (tid < 2) s_cnt_corner[tid] = 0;
-  int issued = 0;                 // store warp, lane 0: tiles handed to the CTA
-  bool producing = true;          // ... tickets not yet exhausted
-  unsigned long long pending = 0; // ... the next ticket, fetched a tile ahead
   if (warp == WSTORE && lane == 0) {
 #pragma unroll
     for (int s = 0; s < S; ++s) {
@@ -142,6 +139,16 @@ __global__ void __launch_bounds__(TileShapeWS<TIn, TOut, A, RPW, NWC, DIRECT, CT
       mbar_init(smem_u32(&s_done[s]), NWC);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+
+  int issued = 0;                 // store warp, lane 0: tiles handed to the CTA
+  bool producing = true;          // ... tickets not yet exhausted
+  unsigned long long pending = 0; // ... the next ticket, fetched a tile ahead
+  if (warp == WSTORE && lane == 0) {
+    // One ticket after the other (the first tiles of all CTAs come before anyone's
+    // second), each a round trip to L2: done before the other roles started, it held the first
+    // tile's sums back to 5.5-9.5 us after the CTA's start at 8192^2.
     for (int s = 0; s < S && producing; ++s) {
       const TilePlan tp = plan_tile<REV>(P, atomicAdd(&P.ws->ticket, 1ull));
       issue_tile<TIn, TW, TH, SH::IN_BYTES>(P, tp, s, stages + s * STAGE_ELEMS, s_tile, s_img, s_tx, s_ty, s_pl,
@@ -151,7 +158,6 @@ __global__ void __launch_bounds__(TileShapeWS<TIn, TOut, A, RPW, NWC, DIRECT, CT
     }
     if (producing) pending = atomicAdd(&P.ws->ticket, 1ull);
   }
-  __syncthreads();
 
   if (DIRECT && warp == WSTORE && lane == 0) {
     // ---- producer thread: each stage is refilled once the output phase of its

@@ -545,7 +545,7 @@ int choose_config_locked(int in_t, int out_t, int mode, int dir, long long w, lo
 
 satgb_status launch_locked(const Variant* v, const ImageDesc* table_dev, const ImageDesc& img0,
                            long long n_images, long long n_tiles, Workspace& ws, int dev,
-                           cudaStream_t s, const unsigned long long* order = nullptr) {
+                           cudaStream_t s, const ulonglong2* order = nullptr) {
   const Layout L = layout_for(n_tiles, v);
   satgb_status st = ensure_ws(ws, L.total, s);
   if (st != SATGB_OK) return st;
@@ -711,7 +711,7 @@ struct BatchSeg {
   double pixels = 0;
   ImageDesc img0;
   ImageDesc* table = nullptr;          // device: the descriptors, then the tile order
-  unsigned long long* order = nullptr; // inside the same allocation (nullptr: images one after the other)
+  ulonglong2* order = nullptr; // inside the same allocation (nullptr: images one after the other)
 };
 
 struct satgb_batch_plan_s {
@@ -1060,8 +1060,8 @@ void seg_free(BatchSeg& g) {
 // of all the images advance together instead of one image after another,
 // whose chains of dependent tiles would otherwise leave most SMs waiting.
 // Empty when a tile coordinate or an image index does not fit the encoding.
-std::vector<unsigned long long> diagonal_order(const std::vector<ImageDesc>& table) {
-  std::vector<unsigned long long> order;
+std::vector<ulonglong2> diagonal_order(const std::vector<ImageDesc>& table) {
+  std::vector<ulonglong2> order;
   if (table.size() >= (1ULL << 24)) return order;
   long long maxd = 0, n = 0;
   for (auto& d : table) {
@@ -1078,13 +1078,15 @@ std::vector<unsigned long long> diagonal_order(const std::vector<ImageDesc>& tab
     }
   std::vector<long long> start(maxd + 1, 0);
   for (long long dd = 1; dd <= maxd; ++dd) start[dd] = start[dd - 1] + count[dd - 1];
-  order.assign(n, 0ull);
+  order.assign(n, ulonglong2{0ull, 0ull});
   for (size_t i = 0; i < table.size(); ++i) {
     const ImageDesc& d = table[i];
     for (long long dd = 0; dd < (long long)d.ntx + d.nty - 1; ++dd) {
       const long long lo = std::max(0LL, dd - (d.ntx - 1)), hi = std::min<long long>(dd, d.nty - 1);
       for (long long ty = lo; ty <= hi; ++ty)
-        order[start[dd]++] = ((unsigned long long)i << 40) | ((unsigned long long)ty << 20) | (unsigned long long)(dd - ty);
+        order[start[dd]++] = ulonglong2{
+            (unsigned long long)(d.tile_base + ty * d.ntx + (dd - ty)),
+            ((unsigned long long)i << 40) | ((unsigned long long)ty << 20) | (unsigned long long)(dd - ty)};
     }
   }
   return order;
@@ -1111,17 +1113,17 @@ satgb_status seg_build(satgb_batch_plan_s* p, int cls, int cfg, cudaStream_t s) 
   g.n_tiles = base;
   if (table.empty()) return SATGB_OK;
   g.img0 = table[0];
-  const std::vector<unsigned long long> order = table.size() > 1 ? diagonal_order(table) : std::vector<unsigned long long>();
+  const std::vector<ulonglong2> order = table.size() > 1 ? diagonal_order(table) : std::vector<ulonglong2>();
   const size_t tbytes = (table.size() * sizeof(ImageDesc) + 255) & ~(size_t)255;
-  if (cudaMalloc(&g.table, tbytes + order.size() * sizeof(unsigned long long)) != cudaSuccess) {
+  if (cudaMalloc(&g.table, tbytes + order.size() * sizeof(ulonglong2)) != cudaSuccess) {
     cudaGetLastError();
     g.table = nullptr;
     return fail(SATGB_ERR_ALLOC, "image table allocation failed");
   }
   cudaError_t e = cudaMemcpyAsync(g.table, table.data(), table.size() * sizeof(ImageDesc), cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess && !order.empty()) {
-    g.order = reinterpret_cast<unsigned long long*>(reinterpret_cast<char*>(g.table) + tbytes);
-    e = cudaMemcpyAsync(g.order, order.data(), order.size() * sizeof(unsigned long long), cudaMemcpyHostToDevice, s);
+    g.order = reinterpret_cast<ulonglong2*>(reinterpret_cast<char*>(g.table) + tbytes);
+    e = cudaMemcpyAsync(g.order, order.data(), order.size() * sizeof(ulonglong2), cudaMemcpyHostToDevice, s);
   }
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return cuda_fail(e, "image table upload");

@@ -704,3 +704,29 @@ def test_stress_16384_compensated_f32(cuda, oracle):
     print(f"\n[precision 16384^2 f32u compensated] {e}")
     assert e["max_rel"] <= 1e-6, e
     assert e["max_rel_abs"] <= TOL_COMP, e
+
+
+@pytest.mark.parametrize("cfg", [0, 1, 2, 5, 6])
+@pytest.mark.parametrize("shape", [(1, 1), (128, 128), (129, 129), (130, 20001), (20001, 130), (1, 70000), (70000, 1),
+                                   (1025, 1153), (2300, 700), (700, 2300), (3000, 2944)])
+def test_tile_orders(cuda, cfg, shape):
+    """Every tile of every order (anti-diagonals of wide, tall and square tile
+    grids, single rows and columns of tiles, row-major) is computed once: u8 -> u32
+    bit for bit, both directions."""
+    h, w = shape
+    g = torch.Generator(device="cpu").manual_seed(h * 7 + w)
+    x = torch.randint(0, 256, (h, w), dtype=torch.uint8, generator=g).to(cuda)
+    try:
+        sat_gb300.set_config(cfg)
+        for rev in (False, True):
+            ref = x.to(torch.int64)
+            if rev:
+                ref = ref.flip((0, 1))
+            ref = ref.cumsum(0).cumsum(1)
+            if rev:
+                ref = ref.flip((0, 1))
+            out = sat_gb300.sat(x, torch.uint32, reverse=rev)
+            assert torch.equal(out.view(torch.int32).to(torch.int64) & 0xFFFFFFFF, ref & 0xFFFFFFFF), rev
+        sat_gb300.stream_check()
+    finally:
+        sat_gb300.set_config(-1)
