@@ -226,6 +226,12 @@ const char* dtype_name(int t) {
 struct Workspace {
   void* base = nullptr;
   size_t bytes = 0;
+  // Padded rows of a staged input (sat_single).  An allocation of their own: a later
+  // launch with more status words would find pixels where its words are to be published, and
+  // four bytes of pixels and padding can equal its tag (a row's last pixel and three
+  // zeros are the tag of one of the first 63 launches).
+  void* stage = nullptr;
+  size_t stage_bytes = 0;
 };
 
 struct Layout {
@@ -280,6 +286,24 @@ satgb_status ensure_ws(Workspace& ws, size_t bytes, cudaStream_t s) {
   }
   ws.base = p;
   ws.bytes = bytes;
+  return SATGB_OK;
+}
+
+satgb_status ensure_stage(Workspace& ws, size_t bytes, cudaStream_t s) {
+  if (ws.stage_bytes >= bytes) return SATGB_OK;
+  bytes = std::max(bytes, ws.stage_bytes + ws.stage_bytes / 2);
+  bytes = (bytes + 4095) & ~(size_t)4095;
+  if (ws.stage) {
+    cudaError_t e = cudaStreamSynchronize(s); // earlier calls may still read it
+    if (e != cudaSuccess) return cuda_fail(e, "cudaStreamSynchronize");
+    ws_free(ws.stage);
+    ws.stage = nullptr;
+    ws.stage_bytes = 0;
+  }
+  void* p = ws_alloc(bytes);
+  if (!p) return fail(SATGB_ERR_ALLOC, "staging allocation of %zu bytes failed", bytes);
+  ws.stage = p;
+  ws.stage_bytes = bytes;
   return SATGB_OK;
 }
 
@@ -639,8 +663,8 @@ satgb_status sat_single(int in_t, int out_t, int mode, int dir, const void* d_in
   if (!v) return fail(SATGB_ERR_UNSUPPORTED_TYPES, "no kernel for %s -> %s mode %d dir %d", dtype_name(in_t), dtype_name(out_t), mode, dir);
   Workspace& ws = g_ws[std::make_pair(dev, (void*)s)];
   // A large image of 1-byte inputs whose rows TMA cannot address (packed rows
-  // of odd widths) is first copied into 16-byte rows behind the look-back words
-  // in the workspace, and the tile kernel reads the copy through TMA: u8 -> u32
+  // of odd widths) is first copied into 16-byte rows in the workspace's
+  // staging buffer, and the tile kernel reads the copy through TMA: u8 -> u32
   // 8191^2 239 -> 158 us, 4095^2 68 -> 59 us.  For wider inputs the copy costs
   // more than it saves (f32 8191^2: 197 us in place against ~220 staged).
   const void* src = d_in;
@@ -649,13 +673,11 @@ satgb_status sat_single(int in_t, int out_t, int mode, int dir, const void* d_in
   bool staged = false;
   if (planes == 1 && in_sz == 1 && width * height >= kStageMinPixels && width >= 16 &&
       !tma_ok(d_in, width, height, in_pitch, 1, 0, in_sz)) {
-    const long long tiles = ((width + v->TW - 1) / v->TW) * ((height + v->TH - 1) / v->TH);
-    const size_t look = (layout_for(tiles, v).total + 255) & ~(size_t)255;
     const size_t pitch = ((size_t)width + 15) & ~(size_t)15;
-    st = ensure_ws(ws, look + pitch * (size_t)height, s);
+    st = ensure_stage(ws, pitch * (size_t)height, s);
     if (st != SATGB_OK) return st;
     job.src = static_cast<const unsigned char*>(d_in);
-    job.dst = static_cast<unsigned char*>(ws.base) + look;
+    job.dst = static_cast<unsigned char*>(ws.stage);
     job.src_pitch = in_pitch;
     job.dst_pitch = (int64_t)pitch;
     job.row_bytes = width;
@@ -841,8 +863,8 @@ satgb_status satgb_reserve(int64_t width, int64_t height, satgb_stream stream) {
   int dev = 0;
   satgb_status st = get_device(&dev);
   if (st != SATGB_OK) return st;
-  // the largest layout over every variant, with the staging rows of a 1-byte
-  // input behind it where a call would stage one (sat_single)
+  // the largest layout over every variant, and the staging rows of a 1-byte
+  // input where a call would stage one (sat_single)
   size_t need = 0;
   const size_t stage = width * height >= kStageMinPixels ? (((size_t)width + 15) & ~(size_t)15) * (size_t)height : 0;
   using ListFn = const Variant* (*)(int*);
@@ -853,11 +875,12 @@ satgb_status satgb_reserve(int64_t width, int64_t height, satgb_stream stream) {
     for (int i = 0; i < n; ++i) {
       long long nt = ((width + v[i].TW - 1) / v[i].TW) * ((height + v[i].TH - 1) / v[i].TH);
       const size_t look = layout_for(nt, &v[i]).total;
-      need = std::max(need, dtype_size(v[i].in_t) == 1 && stage ? ((look + 255) & ~(size_t)255) + stage : look);
+      need = std::max(need, look);
     }
   }
   Workspace& ws = g_ws[std::make_pair(dev, (void*)stream)];
-  return ensure_ws(ws, need, (cudaStream_t)stream);
+  st = ensure_ws(ws, need, (cudaStream_t)stream);
+  return st == SATGB_OK && stage ? ensure_stage(ws, stage, (cudaStream_t)stream) : st;
 }
 
 satgb_status satgb_stream_check(satgb_stream stream) {
@@ -890,7 +913,10 @@ satgb_status satgb_stream_check(satgb_stream stream) {
 satgb_status satgb_release(void) {
   std::lock_guard<std::mutex> lk(g_mu);
   cudaDeviceSynchronize();
-  for (auto& kv : g_ws) ws_free(kv.second.base);
+  for (auto& kv : g_ws) {
+    ws_free(kv.second.base);
+    if (kv.second.stage) ws_free(kv.second.stage);
+  }
   g_ws.clear();
   g_desc_cache.clear();
   return SATGB_OK;

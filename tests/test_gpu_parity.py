@@ -730,3 +730,29 @@ def test_tile_orders(cuda, cfg, shape):
         sat_gb300.stream_check()
     finally:
         sat_gb300.set_config(-1)
+
+
+def test_staged_pixels_are_never_status_words(cuda):
+    """A staged image leaves its padded rows in the stream's workspace: launches with
+    more status words than the staged one had must not take pixels for published sums.  A fresh
+    stream's first launches carry small tags, and where a row ends two bytes before a
+    16-byte group's second half a pixel followed by zeros looks like one: every pixel value
+    stands there in some row."""
+    h, w = 2049, 2051
+    flat = (torch.arange(h * w + 16) * 2654435761 // 65536 % 256).to(torch.uint8).to(cuda)
+    x = flat[1:1 + h * w].view(h, w)
+    big = torch.randint(0, 256, (4100, 8208), dtype=torch.uint8, device=cuda)
+    ref = big.to(torch.int64).cumsum(0).cumsum(1)
+    torch.cuda.synchronize()
+    s = torch.cuda.Stream()
+    try:
+        with torch.cuda.stream(s):
+            for cfg in (0, 2, 5):
+                for _ in range(3):
+                    sat_gb300.set_config(6)
+                    sat_gb300.sat(x, torch.uint32)
+                    sat_gb300.set_config(cfg)
+                    out = sat_gb300.sat(big, torch.uint32)
+                    assert torch.equal(out.view(torch.int32).to(torch.int64) & 0xFFFFFFFF, ref & 0xFFFFFFFF), cfg
+    finally:
+        sat_gb300.set_config(-1)
