@@ -5,6 +5,7 @@
 #include "sat_kernel.cuh"
 #include "sat_kernel_r.cuh"
 #include "sat_kernel_ws.cuh"
+#include "sat_kernel_wd.cuh"
 #include "sat_kernel_rm.cuh"
 #include "sat_registry.h"
 
@@ -121,6 +122,47 @@ Variant make_variant_ws(int in_t, int out_t, int mode, int cfg) {
                  SH::TH, SH::TW, Ar<A>::K, SH::THREADS, SH::DYN_SMEM};
 }
 
+// The same three for sat_tile_kernel_wd (1-byte inputs, 4-byte sums).
+template <class TIn, class TOut, class A, bool REV>
+cudaError_t prepare_impl_wd() {
+  using SH = TileShapeWD<TIn, TOut, A>;
+  constexpr int kMaxDev = 64;
+  static std::atomic<int> done[kMaxDev];
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev >= 0 && dev < kMaxDev && done[dev].load(std::memory_order_acquire)) return cudaSuccess;
+  e = cudaFuncSetAttribute(&sat_tile_kernel_wd<TIn, TOut, A, REV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           SH::DYN_SMEM);
+  if (e == cudaSuccess && dev >= 0 && dev < kMaxDev) done[dev].store(1, std::memory_order_release);
+  return e;
+}
+
+template <class TIn, class TOut, class A, bool REV>
+cudaError_t launch_impl_wd(const SatParams& p, int grid, cudaStream_t s) {
+  using SH = TileShapeWD<TIn, TOut, A>;
+  cudaError_t e = prepare_impl_wd<TIn, TOut, A, REV>();
+  if (e != cudaSuccess) return e;
+  sat_tile_kernel_wd<TIn, TOut, A, REV><<<grid, SH::THREADS, SH::DYN_SMEM, s>>>(p);
+  return cudaGetLastError();
+}
+
+// Configuration 5: the packed kernel for 1-byte inputs with 4-byte sums, sat_tile_kernel_ws with direct
+// stores for every other accumulator.
+template <class TIn, class TOut, class A, bool REV>
+Variant make_variant_5(int in_t, int out_t, int mode) {
+  if constexpr (sizeof(TIn) == 1 && sizeof(A) == 4) {
+    using SH = TileShapeWD<TIn, TOut, A>;
+    return Variant{in_t, out_t, mode, REV ? 1 : 0, 5,
+                   &launch_impl_wd<TIn, TOut, A, REV>,
+                   &prepare_impl_wd<TIn, TOut, A, REV>,
+                   (const void*)&sat_tile_kernel_wd<TIn, TOut, A, REV>,
+                   SH::TH, SH::TW, Ar<A>::K, SH::THREADS, SH::DYN_SMEM};
+  } else {
+    return make_variant_ws<TIn, TOut, A, REV, 8, sizeof(A) == 8 ? 8 : 16, true>(in_t, out_t, mode, 5);
+  }
+}
+
 // The same three for sat_tile_kernel_rm (row-major tile order, direct stores).
 template <class TIn, class TOut, class A, bool REV, int RPW, int NWC>
 cudaError_t prepare_impl_rm() {
@@ -190,7 +232,7 @@ Variant make_variant_rm(int in_t, int out_t, int mode, int cfg) {
       satgb::make_variant<TIN, TOUT, A, REV, SG_CFG1_RPW(A), 16, 1>(IT, OT, MODE, 1),    \
       satgb::make_variant<TIN, TOUT, A, REV, SG_R0_RPW(A), 8, 2>(IT, OT, MODE, 2),       \
       satgb::make_variant_r<TIN, TOUT, A, REV, 8, 16, 1>(IT, OT, MODE, 3),               \
-      satgb::make_variant_ws<TIN, TOUT, A, REV, 8, SG_WS_NWC(A), true>(IT, OT, MODE, 5),   \
+      satgb::make_variant_5<TIN, TOUT, A, REV>(IT, OT, MODE),                              \
       satgb::make_variant_rm<TIN, TOUT, A, REV, 8, SG_WS_NWC(A)>(IT, OT, MODE, 6)
 #define SG_ALL(TIN, TOUT, A, IT, OT, MODE) \
   SG_DIR(TIN, TOUT, A, IT, OT, MODE, false), SG_DIR(TIN, TOUT, A, IT, OT, MODE, true)

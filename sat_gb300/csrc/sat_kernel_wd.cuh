@@ -1,0 +1,481 @@
+// sat_kernel_wd.cuh -- the warp-specialized tile loop for 1-byte inputs with 4-byte sums
+// (configuration 5 for those pairs).
+//
+// A tile's data flow is that of sat_kernel_ws.cuh with direct stores.  What bounds that kernel for 8-bit
+// pixels is not memory (u8 -> u32 8192^2: 99.7 us, floor 49.5): with its stores left out it is as
+// slow, since its compute warps add pixel by pixel, and a tile's carries have one tile period to arrive
+// in, while an SM stores 25 bytes a cycle at most, the 64 KB of a tile's results are 1.4 us of
+// that, and the look-backs' loads queue behind them.  Three things differ here (82.7 us at 8192^2, 30.9 at
+// 4096^2 for 33.5; 70.4 with look-backs that find everything published, 57.9 without stores on top).
+//
+// Arithmetic.  A tile's own sums of 8-bit pixels are small integers, so the compute warps work
+// on the packed words: a row's four pixels a lane are added with one dp4a, column sums
+// and the lanes' row totals go two to a register in 16 bits (128 columns of 255 are
+// 32,640), a warp reduction is one instruction for two rows, and each output's row prefix is
+// one dp4a on top of its base.  Signed pixels are biased by 128 where sums are packed.
+//
+// Depth.  Each 16 KB stage leaves room for many: the sums of tile k+3 are taken before the results of
+// tile k are stored (kWdDepth sets of the shared vectors), so carries have three tile
+// periods (8192^2: depth 3 88.7 us, 4 82.7, 5 and 6 82.6 to 82.8).
+//
+// Roles.  Publishing waits for no other tile: the compute warps publish the rows' sums as they take
+// them, the summing warps the columns', and the resolving warps, which walk row j's and column j's
+// look-back side by side, are warps of their own; the corner's look-back has another.  With one group
+// of warps that published, walked the rows and walked the columns in turn, a tile that waited
+// held back the aggregates of the next (101 us at depth 2).
+#pragma once
+#include "sat_kernel_ws.cuh"
+
+namespace satgb {
+
+constexpr int kWdDepth = 4; // sets of the shared vectors: the tile in output and three whose sums are out
+// named barriers, one a set: partials in, sums in, carries in; the resolving warps' own
+constexpr int kWdAgg0 = 1, kWdSum0 = 1 + kWdDepth, kWdCar0 = 1 + 2 * kWdDepth, kWdRows = 1 + 3 * kWdDepth;
+static_assert(kWdRows < 16, "named barriers");
+
+// One more round of a wait; false (an error recorded) when it has to give up.
+struct WordWait {
+  uint32_t round = 0;
+  unsigned long long t0 = 0;
+  __device__ __forceinline__ bool again(const SatParams& P, long long tile) {
+    if (round == 0) t0 = global_timer_ns();
+    if ((++round & 15u) == 0u &&
+        ((long long)(global_timer_ns() - t0) > P.wait_limit_ns || ld_relaxed_u32(&P.ws->error) != 0u)) {
+      record_error(P, tile);
+      return false;
+    }
+    return true;
+  }
+};
+
+template <class TIn, class TOut, class A>
+struct TileShapeWD {
+  static constexpr int CPT = 4, RPW = 8, NWC = 16;
+  static constexpr int TW = 128, TH = NWC * RPW;
+  static constexpr int NPW = TW / 32, NVW = 4, NRW = TH / 32; // summing, resolving warps (and of them, with rows)
+  static constexpr int STAGE_BYTES = TH * TW;
+  static constexpr int STATIC_BYTES = (kWdDepth * (NWC * TW + TH + 2 * TW + TH + NWC + NRW + 4)) * 4 + 512;
+  static constexpr int S = Stages<STAGE_BYTES, STATIC_BYTES, 1>::value;
+  static constexpr int DYN_SMEM = S * STAGE_BYTES;
+  static constexpr int THREADS = (NWC + NPW + NVW + 2) * 32;
+};
+
+// The sum of a word's four pixels picked by the mask's bytes (0 or 1), plus c.
+template <class TIn>
+__device__ __forceinline__ uint32_t pixel_sum(uint32_t w, uint32_t mask, uint32_t c) {
+  if constexpr (sizeof(TIn) == 1 && TIn(-1) < TIn(0)) return (uint32_t)__dp4a((int)w, (int)mask, (int)c);
+  else return __dp4a(w, mask, c);
+}
+
+// A small integer (|v| < 2^22) as the accumulator.
+template <class A>
+__device__ __forceinline__ A small_int(uint32_t v) {
+  if constexpr (sizeof(A) == 4 && A(0.5f) != A(0)) return __uint_as_float(0x4B400000u + v) - 12582912.0f; // exact
+  else return v;
+}
+
+template <class TIn, class TOut, class A, bool REV>
+__global__ void __launch_bounds__(TileShapeWD<TIn, TOut, A>::THREADS, 1)
+    sat_tile_kernel_wd(const __grid_constant__ SatParams P) {
+  using SH = TileShapeWD<TIn, TOut, A>;
+  constexpr int CPT = SH::CPT, RPW = SH::RPW, NWC = SH::NWC;
+  constexpr int TW = SH::TW, TH = SH::TH, S = SH::S;
+  constexpr int NPW = SH::NPW, NVW = SH::NVW, NRW = SH::NRW;
+  constexpr int WSUM = NWC, WRES = NWC + NPW, WCOR = WRES + NVW, WSTORE = WCOR + 1; // first warp of each role
+  constexpr int NAGG = (NWC + NPW) * 32;     // compute + summing warps
+  constexpr int NSUM = (NPW + NVW) * 32;     // summing + resolving warps
+  constexpr int NCAR = (NWC + NVW + 1) * 32; // compute + resolving + corner warps
+  constexpr bool SIGNED = TIn(-1) < TIn(0);
+  constexpr uint32_t kBias = SIGNED ? 128u : 0u;
+  static_assert(S > kWdDepth, "stages for the tile in output, those whose sums are out and one loading");
+  static_assert(NRW == NVW && NPW == NVW, "a resolving thread has one row and one column");
+  constexpr int K = 1;
+  using AR = Ar<A>;
+
+  extern __shared__ __align__(128) unsigned char dsmem[];
+  TIn* stages = reinterpret_cast<TIn*>(dsmem);
+
+  __shared__ A s_colp[kWdDepth][NWC][TW];   // column partials a warp (by slot), then their exclusive prefix over the warps
+  __shared__ A s_rowagg[kWdDepth][TH];      // row totals
+  __shared__ A s_colagg[kWdDepth][TW];      // column sums (by slot)
+  __shared__ A s_colabove[kWdDepth][TW];    // column look-back results (by slot)
+  __shared__ A s_rowleft[kWdDepth][TH];     // row look-back results
+  __shared__ A s_rlprev[kWdDepth][NWC];     // per compute warp: sum of rowleft over the rows before it (scan order)
+  __shared__ A s_rwt[kWdDepth][NRW];        // resolving warps: sum of rowleft over each warp's 32 rows
+  __shared__ A s_corner[kWdDepth], s_u[kWdDepth];
+  __shared__ int s_uready[kWdDepth];  // k + 1 once tile k's u is in s_u
+  __shared__ long long s_tile[S];    // spatial tile index per stage (-1: no more tiles)
+  __shared__ int s_img[S];
+  __shared__ int s_tx[S], s_ty[S], s_pl[S];
+  __shared__ __align__(8) unsigned long long s_full[S];
+  __shared__ __align__(8) unsigned long long s_done[S]; // the stage has been read and may be refilled
+
+  const int tid = threadIdx.x;
+  const int lane = tid & 31;
+  const int warp = tid >> 5;
+  const uint32_t epoch = ld_relaxed_u32(&P.ws->epoch);
+  const uint32_t tagA = make_tag(epoch, kStateAgg);
+  const uint32_t tagI = make_tag(epoch, kStateInc);
+
+  if (tid < kWdDepth) s_uready[tid] = 0;
+  if (warp == WSTORE && lane == 0) {
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+      mbar_init(smem_u32(&s_full[s]), 1);
+      mbar_init(smem_u32(&s_done[s]), NWC);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+
+  if (warp == WSTORE && lane == 0) {
+    // ---- producer thread: fills the stages, then refills each once the output phase of its
+    //      tile has read it; a ticket is fetched a tile ahead ---------------------------
+    bool producing = true;
+    for (int s = 0; s < S && producing; ++s) {
+      const TilePlan tp = plan_tile<REV>(P, atomicAdd(&P.ws->ticket, 1ull));
+      issue_tile<TIn, TW, TH, SH::STAGE_BYTES>(P, tp, s, stages + s * SH::STAGE_BYTES, s_tile, s_img, s_tx, s_ty, s_pl,
+                                              s_full);
+      producing = tp.t >= 0;
+    }
+    unsigned long long pending = producing ? atomicAdd(&P.ws->ticket, 1ull) : 0ull;
+    for (int k = 0; producing; ++k) {
+      const TilePlan next = plan_tile<REV>(P, pending);
+      if (next.t >= 0) pending = atomicAdd(&P.ws->ticket, 1ull);
+      const int st = k % S;
+      mbar_wait_bounded(smem_u32(&s_done[st]), (k / S) & 1, P, -1);
+      issue_tile<TIn, TW, TH, SH::STAGE_BYTES>(P, next, st, stages + st * SH::STAGE_BYTES, s_tile, s_img, s_tx, s_ty,
+                                              s_pl, s_full);
+      producing = next.t >= 0;
+    }
+  }
+
+  if (warp < NWC) {
+    // ---- compute warps ----------------------------------------------------------
+    // The sums of tile kk: false when the tickets ran out (the summing warps still get their
+    // AGG arrival, to see the end).
+    auto sums = [&](int kk) -> bool {
+      const int st = kk % S, kb = kk % kWdDepth;
+      mbar_wait_bounded(smem_u32(&s_full[st]), (kk / S) & 1, P, -1);
+      const bool have = s_tile[st] >= 0;
+      if (have) {
+        const ImageView D = image_view(P, s_img[st]);
+        const long long x0 = (long long)s_tx[st] * TW, y0 = (long long)s_ty[st] * TH;
+        const long long xt = x0 + (long long)lane * CPT;
+        const long long rem = D.width - xt;
+        const int nvalid = rem <= 0 ? 0 : (rem >= CPT ? CPT : (int)rem);
+        TIn* sb = stages + st * SH::STAGE_BYTES + (warp * RPW) * TW + lane * CPT;
+        const bool tma = D.flags & kInTma;
+        if (!tma || (nvalid > 0 && xt + nvalid > D.tma_in_w)) {
+          // no TMA for this image, or columns past the map (they arrived as zeros)
+          const TIn* gin = static_cast<const TIn*>(D.in) + (long long)s_pl[st] * D.in_plane +
+                           (y0 + warp * RPW) * D.in_pitch + xt;
+          const long long rows = D.height - (y0 + warp * RPW);
+          const int c0 = tma ? (int)(D.tma_in_w - xt > 0 ? D.tma_in_w - xt : 0) : 0;
+          stage_fill<TIn, CPT, RPW, TW>(sb, gin, D.in_pitch, rows < 0 ? 0 : (rows > RPW ? RPW : (int)rows), nvalid,
+                                        c0, (D.flags & kInVec) != 0);
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); // before TMA refills the stage
+        }
+        uint32_t even = 0, odd = 0; // columns 0, 2 and 1, 3 over the rows, 16 bits each
+        uint32_t t[RPW / 2];        // the lane's row totals, rows 2i and 2i + 1
+#pragma unroll
+        for (int r = 0; r < RPW; ++r) {
+          const uint32_t w = *reinterpret_cast<const uint32_t*>(sb + r * TW);
+          const uint32_t b = SIGNED ? w ^ 0x80808080u : w;
+          even += b & 0x00ff00ffu;
+          odd += (b >> 8) & 0x00ff00ffu;
+          const uint32_t s = __dp4a(b, 0x01010101u, 0u);
+          if (r & 1) t[r / 2] += s << 16;
+          else t[r / 2] = s;
+        }
+        s_colp[kb][warp][0 * 32 + lane] = small_int<A>((even & 0xffffu) - RPW * kBias);
+        s_colp[kb][warp][1 * 32 + lane] = small_int<A>((odd & 0xffffu) - RPW * kBias);
+        s_colp[kb][warp][2 * 32 + lane] = small_int<A>((even >> 16) - RPW * kBias);
+        s_colp[kb][warp][3 * 32 + lane] = small_int<A>((odd >> 16) - RPW * kBias);
+        uint32_t mine = 0;
+#pragma unroll
+        for (int i = 0; i < RPW / 2; ++i) {
+          const uint32_t s = __reduce_add_sync(0xffffffffu, t[i]);
+          if (lane >> 1 == i) mine = lane & 1 ? s >> 16 : s & 0xffffu;
+        }
+        if (lane < RPW) {
+          const A sum = small_int<A>(mine - TW * kBias);
+          const int y = warp * RPW + lane, lx = REV ? D.ntx - 1 - s_tx[st] : s_tx[st];
+          s_rowagg[kb][y] = sum;
+          if (lx < D.ntx - 1 && s_tile[st] != P.stall_tile)
+            publish<A>(P.row_words + ((unsigned long long)s_tile[st] * TH + y) * K, sum, tagA);
+        }
+      }
+      named_arrive(kWdAgg0 + kb, NAGG);
+      return have;
+    };
+
+    // ahead[i]: tile k + i exists
+    bool ahead[kWdDepth];
+    ahead[0] = sums(0);
+#pragma unroll
+    for (int i = 1; i < kWdDepth - 1; ++i) ahead[i] = ahead[i - 1] && sums(i);
+    for (int k = 0; ahead[0]; ++k) {
+      ahead[kWdDepth - 1] = ahead[kWdDepth - 2] && sums(k + kWdDepth - 1);
+      const int st = k % S, kb = k % kWdDepth;
+      named_sync(kWdCar0 + kb, NCAR); // tile k's carries are in
+
+      // ---- output phase of tile k -----------------------------------------------
+      const ImageView D = image_view(P, s_img[st]);
+      const uint32_t flags = D.flags;
+      const long long x0 = (long long)s_tx[st] * TW, y0 = (long long)s_ty[st] * TH;
+      const long long xt = x0 + (long long)lane * CPT;
+      const long long rem = D.width - xt;
+      const int nvalid = rem <= 0 ? 0 : (rem >= CPT ? CPT : (int)rem);
+      const TIn* sb = stages + st * SH::STAGE_BYTES + (warp * RPW) * TW + lane * CPT;
+      uint32_t w[RPW];
+#pragma unroll
+      for (int r = 0; r < RPW; ++r) w[r] = *reinterpret_cast<const uint32_t*>(sb + r * TW);
+      __syncwarp();
+      TOut* out = static_cast<TOut*>(D.out) + (long long)s_pl[st] * D.out_plane + (y0 + warp * RPW) * D.out_pitch + xt;
+      const long long left = D.height - (y0 + warp * RPW);
+      const int rows = left < 0 ? 0 : (left > RPW ? RPW : (int)left);
+      if (lane == 0) mbar_arrive(smem_u32(&s_done[st])); // the stage goes back to the producer
+      // the lanes' exclusive row prefixes, two rows a register: inclusive scans less the lane's own total
+      uint32_t ex[RPW / 2];
+#pragma unroll
+      for (int i = 0; i < RPW / 2; ++i) {
+        const uint32_t lo = __dp4a(SIGNED ? w[2 * i] ^ 0x80808080u : w[2 * i], 0x01010101u, 0u);
+        const uint32_t hi = __dp4a(SIGNED ? w[2 * i + 1] ^ 0x80808080u : w[2 * i + 1], 0x01010101u, 0u);
+        ex[i] = lo + (hi << 16);
+      }
+      uint32_t own[RPW / 2];
+#pragma unroll
+      for (int i = 0; i < RPW / 2; ++i) own[i] = ex[i];
+      A top[CPT], cp[CPT];
+#pragma unroll
+      for (int i = 0; i < CPT; ++i) {
+        const int c = REV ? CPT - 1 - i : i;
+        cp[c] = AR::add(s_colabove[kb][c * 32 + lane], s_colp[kb][warp][c * 32 + lane]);
+        if (i) cp[c] = AR::add(cp[REV ? c + 1 : c - 1], cp[c]);
+      }
+      A incl = cp[REV ? 0 : CPT - 1];
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const A o = REV ? AR::shfl_down(incl, d) : AR::shfl_up(incl, d);
+        const bool in = REV ? (lane + d < 32) : (lane >= d);
+        uint32_t e[RPW / 2];
+#pragma unroll
+        for (int i = 0; i < RPW / 2; ++i)
+          e[i] = REV ? __shfl_down_sync(0xffffffffu, ex[i], d) : __shfl_up_sync(0xffffffffu, ex[i], d);
+        if (in) {
+          incl = AR::add(o, incl);
+#pragma unroll
+          for (int i = 0; i < RPW / 2; ++i) ex[i] += e[i];
+        }
+      }
+      {
+        A e = REV ? AR::shfl_down(incl, 1) : AR::shfl_up(incl, 1);
+        if (lane == (REV ? 31 : 0)) e = AR::zero();
+        const A base = AR::add(AR::add(s_corner[kb], s_rlprev[kb][warp]), e);
+#pragma unroll
+        for (int c = 0; c < CPT; ++c) top[c] = AR::add(base, cp[c]);
+      }
+      const bool vout = (flags & kOutVec) && nvalid == CPT;
+      const uint32_t unbias = (uint32_t)(REV ? 31 - lane : lane) * (4u * kBias);
+#pragma unroll
+      for (int i = 0; i < RPW; ++i) {
+        const int r = REV ? RPW - 1 - i : i;
+        const uint32_t pair = ex[r / 2] - own[r / 2]; // no borrow between the halves: each total is in its sum
+        const uint32_t e = (r & 1 ? pair >> 16 : pair & 0xffffu) - unbias;
+        const A rl = s_rowleft[kb][warp * RPW + r];
+        TOut o[CPT];
+#pragma unroll
+        for (int c = 0; c < CPT; ++c) {
+          const uint32_t mask = REV ? 0x01010101u << (8 * c) : 0x01010101u >> (8 * (CPT - 1 - c));
+          A run;
+          if constexpr (sizeof(A) == 4 && A(0.5f) != A(0))
+            run = AR::add(rl, __uint_as_float(pixel_sum<TIn>(w[r], mask, e + 0x4B400000u)) - 12582912.0f);
+          else run = pixel_sum<TIn>(w[r], mask, e + rl);
+          top[c] = AR::add(top[c], run);
+          o[c] = OutCvt<TOut, A>::out(top[c]);
+        }
+        if (r < rows && nvalid > 0) store_seg<TOut, CPT>(out + r * D.out_pitch, vout, nvalid, o);
+      }
+#pragma unroll
+      for (int i = 0; i + 1 < kWdDepth; ++i) ahead[i] = ahead[i + 1];
+    }
+  }
+
+  if (warp >= WSUM && warp < WRES) {
+    // ---- summing warps: one column (slot) per thread; they wait for no other tile ------------------
+    const int j = tid - WSUM * 32;
+    for (int k = 0;; ++k) {
+      const int st = k % S;
+      mbar_wait_bounded(smem_u32(&s_full[st]), (k / S) & 1, P, -1);
+      const long long t = s_tile[st];
+      named_sync(kWdAgg0 + k % kWdDepth, NAGG); // tile k's partials are in (or there is no tile k)
+      if (t < 0) break;
+      const int kb = k % kWdDepth;
+      const ImageView D = image_view(P, s_img[st]);
+      const int ly = REV ? D.nty - 1 - s_ty[st] : s_ty[st];
+      // the column's partials of every compute warp: all loads first, then the
+      // exclusive prefix over the warps (scan order) and the column sum
+      A v[NWC];
+#pragma unroll
+      for (int w = 0; w < NWC; ++w) v[w] = s_colp[kb][w][j];
+      A run = AR::zero();
+#pragma unroll
+      for (int i = 0; i < NWC; ++i) {
+        const int w = REV ? NWC - 1 - i : i;
+        s_colp[kb][w][j] = run;
+        run = AR::add(run, v[w]);
+      }
+      s_colagg[kb][j] = run;
+      if (ly < D.nty - 1 && t != P.stall_tile)
+        publish<A>(P.col_words + ((unsigned long long)t * TW + j) * K, run, tagA);
+      named_arrive(kWdSum0 + kb, NSUM);
+    }
+  }
+
+  if (warp >= WRES && warp < WCOR) {
+    // ---- resolving warps: row j and column (slot) j per thread -------------------------
+    const int j = tid - WRES * 32;
+    const int rw = warp - WRES;
+    constexpr int D1 = REV ? 1 : -1; // towards the tiles before
+    for (int k = 0;; ++k) {
+      const int st = k % S;
+      mbar_wait_bounded(smem_u32(&s_full[st]), (k / S) & 1, P, -1);
+      const long long t = s_tile[st];
+      if (t < 0) break;
+      const int kb = k % kWdDepth;
+      const ImageView D = image_view(P, s_img[st]);
+      const int ntx = D.ntx, nty = D.nty;
+      const int lx = REV ? ntx - 1 - s_tx[st] : s_tx[st], ly = REV ? nty - 1 - s_ty[st] : s_ty[st];
+      const bool live = t != P.stall_tile;
+      unsigned long long* rbase = P.row_words + ((unsigned long long)t * TH + j) * K;
+      unsigned long long* cbase = P.col_words + ((unsigned long long)t * TW + j) * K;
+      const long long rstep = D1 * (long long)TH * K, cstep = D1 * (long long)ntx * TW * K;
+      EarlyWin<A> wr, wc;
+      early_read<A>(wr, rbase, rstep, lx);
+      early_read<A>(wc, cbase, cstep, ly);
+      named_sync(kWdSum0 + kb, NSUM); // tile k's own sums are in
+      // the row's and the column's look-back side by side: every round walks both windows as far as they
+      // reach and reads again what is still open
+      A left = AR::zero(), above = AR::zero();
+      int ri = 0, ci = 0; // predecessors accounted for
+      bool rdone = lx == 0, cdone = ly == 0;
+      if (rdone && lx < ntx - 1 && live) publish<A>(rbase, s_rowagg[kb][j], tagI);
+      if (cdone && ly < nty - 1 && live) publish<A>(cbase, s_colagg[kb][j], tagI);
+      unsigned long long t0 = 0;
+      for (uint32_t round = 0; !(rdone && cdone); ++round) {
+        bool moved = false;
+        if (!rdone) {
+#pragma unroll
+          for (int q = 0; q < EarlyWin<A>::W; ++q) {
+            A val;
+            const uint32_t state = rdone ? 0u : decode_word<A>(wr.w[q], tagA, tagI, val);
+            if (!state) break;
+            left = AR::add(val, left);
+            ++ri;
+            moved = true;
+            rdone = state == kStateInc || ri >= lx;
+          }
+          if (rdone && lx < ntx - 1 && live) publish<A>(rbase, AR::add(left, s_rowagg[kb][j]), tagI);
+        }
+        if (!cdone) {
+#pragma unroll
+          for (int q = 0; q < EarlyWin<A>::W; ++q) {
+            A val;
+            const uint32_t state = cdone ? 0u : decode_word<A>(wc.w[q], tagA, tagI, val);
+            if (!state) break;
+            above = AR::add(val, above);
+            ++ci;
+            moved = true;
+            cdone = state == kStateInc || ci >= ly;
+          }
+          if (cdone && ly < nty - 1 && live) publish<A>(cbase, AR::add(above, s_colagg[kb][j]), tagI);
+        }
+        if (rdone && cdone) break;
+        if (!moved) {
+          if (t0 == 0) t0 = global_timer_ns();
+          __nanosleep(64);
+          if ((round & 15u) == 15u &&
+              ((long long)(global_timer_ns() - t0) > P.wait_limit_ns || ld_relaxed_u32(&P.ws->error) != 0u)) {
+            record_error(P, t);
+            break;
+          }
+        }
+        if (!rdone) early_read<A>(wr, rbase, rstep, lx, ri);
+        if (!cdone) early_read<A>(wc, cbase, cstep, ly, ci);
+      }
+      s_colabove[kb][j] = above;
+      s_rowleft[kb][j] = left;
+      // inclusive scan of rowleft over the tile's rows, in scan order: within
+      // the warp, then across the warps
+      A incl = left;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const A o = REV ? AR::shfl_down(incl, d) : AR::shfl_up(incl, d);
+        if (REV ? (lane + d < 32) : (lane >= d)) incl = AR::add(o, incl);
+      }
+      if (lane == (REV ? 0 : 31)) s_rwt[kb][rw] = incl;
+      named_sync(kWdRows, NRW * 32);
+      A before = AR::zero();
+#pragma unroll
+      for (int i = 0; i < NRW; ++i) {
+        const int w = REV ? NRW - 1 - i : i;
+        if (REV ? (w > rw) : (w < rw)) before = AR::add(before, s_rwt[kb][w]);
+      }
+      incl = AR::add(before, incl);
+      // rowleft summed over the rows before compute warp w (scan order)
+      if (!REV && (j + 1) % RPW == 0 && j + 1 < TH) s_rlprev[kb][(j + 1) / RPW] = incl;
+      if (REV && j % RPW == 0 && j > 0) s_rlprev[kb][j / RPW - 1] = incl;
+      if (j == (REV ? TH - 1 : 0)) s_rlprev[kb][REV ? NWC - 1 : 0] = AR::zero();
+      if (j == (REV ? 0 : TH - 1)) {
+        vstore(&s_u[kb], incl); // u
+        if (live && ly < nty - 1)
+          publish<A>(P.corner_words + (unsigned long long)t * K, incl, tagA);
+        __threadfence_block();
+        vstore(&s_uready[kb], k + 1);
+      }
+      __syncwarp();
+      named_arrive(kWdCar0 + kb, NCAR);
+    }
+  }
+
+  if (warp == WCOR) {
+    // ---- corner warp: lane 0 ----------------------------------------------------------
+    constexpr int D1 = REV ? 1 : -1;
+    for (int k = 0;; ++k) {
+      const int st = k % S;
+      mbar_wait_bounded(smem_u32(&s_full[st]), (k / S) & 1, P, -1);
+      const long long t = s_tile[st];
+      if (t < 0) break;
+      const int kb = k % kWdDepth;
+      const ImageView D = image_view(P, s_img[st]);
+      const int nty = D.nty, ly = REV ? nty - 1 - s_ty[st] : s_ty[st];
+      unsigned long long* base = P.corner_words + (unsigned long long)t * K;
+      A corner = AR::zero();
+      if (lane == 0) {
+        const long long step = D1 * (long long)D.ntx * K;
+        EarlyWin<A> w[1];
+        early_read<A>(w[0], base, step, ly);
+        A c1[1];
+        resolve_n<A, 1>(w, base, 0, step, ly, tagA, tagI, P, t, c1);
+        corner = c1[0];
+        // u of tile k: the resolving warps have it after every compute warp took tile k's sums, and so is done
+        // with the set's last tile (nothing else keeps this warp from running ahead of them)
+        WordWait wait;
+        while (vload(&s_uready[kb]) != k + 1 && wait.again(P, t)) {
+        }
+        __threadfence_block();
+        s_corner[kb] = corner;
+        if (t != P.stall_tile && ly < nty - 1) publish<A>(base, AR::add(corner, vload(&s_u[kb])), tagI);
+      }
+      __syncwarp();
+      named_arrive(kWdCar0 + kb, NCAR);
+    }
+  }
+
+  // ---- end of launch: the last CTA resets the ticket and advances the epoch --
+  __syncthreads();
+  if (tid == 0) finish_launch(P, epoch);
+}
+
+}  // namespace satgb

@@ -520,9 +520,12 @@ int sms_of(int dev) {
 // 5) once there are at least 4 tiles of 128 x 128 per SM (f32: 2959 vs 2851
 // GB/s at 4096^2, 4521 vs 3893 at 8192^2, 5510 vs 4370 at 16384^2), else the
 // 128-row pipelined tiles (1494 vs 1369 GB/s at 2048^2).
-// 1-byte inputs with 4-byte sums: configuration 5 from 16 tiles per SM (3185
-// vs 3093 GB/s at 8192^2, 4022 vs 3518 at 16384^2, 4358 vs 3621 at 32768^2),
-// the 256-row direct-store tiles below that (2159 vs 2051 at 4096^2).
+// 1-byte inputs with 4-byte sums: the packed kernel of configuration 5 from 3
+// tiles per SM of one plane (u8 -> u32, us: 3072^2 20.8, the row-major kernel
+// 22.5 and the 256-row direct-store tiles 24.7; 4096^2 27.6, 36.0, 33.0; 8192^2
+// 79.3, 210, 102; packed rows 2999 x 3001 31.6, 34.6, 37.1), below that the row-major
+// kernel (2048^2 14.4, configuration 5 16.4; 1024^2 9.9, 11.4), stacks of small
+// planes the 256-row tiles.
 // Compensated f32: the 128-row register tiles (2474 vs 1570 GB/s for
 // configuration 5 at 8192^2, 1096 vs 911 for the 64-row tiles at 2048^2).
 // f64 outputs (slow FP64 adds on GB300): the warp-specialized tiles, whose
@@ -547,10 +550,10 @@ int default_config(long long width, long long height, int sms, int in_sz, int ou
   // 12.9); stacks of small planes stay on configuration 1.
   const bool single = planes <= 1;
   if (in_sz == 1) {
-    if (plane_tiles >= 16LL * sms) return 5;
-    if (single && plane_tiles < 3LL * sms) return 6;
+    if (plane_tiles >= 3LL * sms) return 5;
+    if (single) return 6;
     if (ntx * ((height + 255) / 256) * std::max(1LL, planes) >= 64) return 4;
-    return single ? 6 : 1;
+    return 1;
   }
   if (plane_tiles >= 4LL * sms) return 5;
   return single ? 6 : 1;
@@ -1062,14 +1065,18 @@ BatchKey batch_key(const satgb_batch_plan_s* p, int cls, int sms) {
                   log2_bucket(std::max(1LL, g.n_images)), p->all_tma ? 1 : 0, sms);
 }
 
-// Untuned choice for a class (GB300, the 512-image u8 batch): large images the
+// Untuned choice for a class: 1-byte images of every size the packed tiles of
+// configuration 5 (u8 -> u32 plans, us, with the small class on configuration 2 when rows
+// go through TMA and 6 when they cannot: 512 images of sides 64..4096 703 for 749
+// and, packed, 1007 for 1023; 512 of 64..512 78 for 91 and 106 for 111; 128 of
+// 64..1024 49 for 56 and 64 for 69).  Otherwise large images the
 // warp-specialized direct-store tiles; small images the 64-row two-CTA tiles
-// when rows go through TMA, the row-major tiles when they cannot (packed rows:
-// 1401 vs 1015 GB/s); f64 outputs and the compensated mode as for one image.
+// when rows go through TMA, the row-major tiles when they cannot; f64 outputs
+// and the compensated mode as for one image.
 int batch_default_config(const satgb_batch_plan_s* p, int cls) {
   if (dtype_size(p->out_t) == 8) return 0;
   if (p->mode == SATGB_MODE_COMPENSATED) return 3;
-  if (cls == 0) return 5;
+  if (cls == 0 || dtype_size(p->in_t) == 1) return 5;
   return p->all_tma ? 2 : 6;
 }
 

@@ -756,3 +756,38 @@ def test_staged_pixels_are_never_status_words(cuda):
                     assert torch.equal(out.view(torch.int32).to(torch.int64) & 0xFFFFFFFF, ref & 0xFFFFFFFF), cfg
     finally:
         sat_gb300.set_config(-1)
+
+
+@pytest.mark.parametrize("pixels", ["random", "lowest", "highest"])
+@pytest.mark.parametrize("pair", [("u8", "u32"), ("u8", "f32"), ("i8", "i32"), ("i8", "f32")])
+def test_packed_sums_of_one_byte_pixels(cuda, pair, pixels):
+    """Configuration 5 adds 1-byte pixels packed two and four to a register: pixels of
+    the type's limits, at tile edges, in more tiles than the grid has CTAs, in rows of one tile and
+    columns of one tile, packed and offset rows, both directions.  Integer sums bit for bit; f32 sums
+    exact while they stay below 2^24 and within 1e-5 of the largest sum beyond
+    (64 x 64 tiles of sums of 128 exact rows at most: 2^-24 x 130 roundings)."""
+    dt = {"u8": torch.uint8, "i8": torch.int8, "u32": torch.uint32, "i32": torch.int32, "f32": torch.float32}
+    t_in, t_out = dt[pair[0]], dt[pair[1]]
+    info = torch.iinfo(t_in)
+    lo, hi = {"random": (info.min, info.max), "lowest": (info.min,) * 2, "highest": (info.max,) * 2}[pixels]
+    g = torch.Generator(device="cpu").manual_seed(11)
+    try:
+        sat_gb300.set_config(5)
+        for h, w, pad in [(1, 1, 0), (127, 129, 0), (128, 128, 0), (129, 127, 5), (100, 9001, 0), (9001, 100, 0),
+                          (128, 40000, 0), (40000, 128, 0), (1281, 4099, 0), (2050, 2049, 15), (64, 130000, 0)]:
+            x = torch.randint(lo, hi + 1, (h, w + pad), dtype=t_in, generator=g).to(cuda)[:, pad // 2: pad // 2 + w]
+            for rev in (False, True):
+                ref = x.to(torch.int64)
+                ref = ref.flip((0, 1)) if rev else ref
+                ref = ref.cumsum(0).cumsum(1)
+                ref = ref.flip((0, 1)) if rev else ref
+                out = sat_gb300.sat(x, t_out, reverse=rev)
+                if t_out == torch.float32:
+                    top = int(ref.abs().max())
+                    assert (out.double() - ref.double()).abs().max().item() <= (0 if top < 2**24 else 1e-5 * top), (h, w, rev)
+                else:
+                    got = out.view(torch.int32).to(torch.int64)
+                    assert torch.equal(got & 0xFFFFFFFF, ref & 0xFFFFFFFF), (h, w, rev)
+        sat_gb300.stream_check()
+    finally:
+        sat_gb300.set_config(-1)
