@@ -58,13 +58,15 @@ class satgb_image(ctypes.Structure):
 
 
 MAX_RADII = 4
+RADIUS_ARRAY = ctypes.c_int * MAX_RADII
+BOX_ARRAY = ctypes.c_void_p * MAX_RADII
 
 
 class satgb_box_desc(ctypes.Structure):
     _fields_ = [("width", ctypes.c_int64), ("height", ctypes.c_int64), ("n_planes", ctypes.c_int64),
                 ("d_sat", ctypes.c_void_p), ("sat_pitch", ctypes.c_int64), ("sat_plane_stride", ctypes.c_int64),
-                ("n_radii", ctypes.c_int), ("radius", ctypes.c_int * MAX_RADII),
-                ("d_box", ctypes.c_void_p * MAX_RADII), ("box_pitch", ctypes.c_int64),
+                ("n_radii", ctypes.c_int), ("radius", RADIUS_ARRAY),
+                ("d_box", BOX_ARRAY), ("box_pitch", ctypes.c_int64),
                 ("box_plane_stride", ctypes.c_int64)]
 
 
