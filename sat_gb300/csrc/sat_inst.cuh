@@ -123,27 +123,34 @@ Variant make_variant_ws(int in_t, int out_t, int mode, int cfg) {
 }
 
 // The same three for sat_tile_kernel_wd (1-byte inputs, 4-byte sums).
+template <class TIn, class TOut, class A, bool REV, bool SKEW>
+cudaError_t prepare_one_wd() {
+  return cudaFuncSetAttribute(&sat_tile_kernel_wd<TIn, TOut, A, REV, SKEW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              TileShapeWD<TIn, TOut, A, SKEW>::DYN_SMEM);
+}
+
 template <class TIn, class TOut, class A, bool REV>
 cudaError_t prepare_impl_wd() {
-  using SH = TileShapeWD<TIn, TOut, A>;
   constexpr int kMaxDev = 64;
   static std::atomic<int> done[kMaxDev];
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   if (dev >= 0 && dev < kMaxDev && done[dev].load(std::memory_order_acquire)) return cudaSuccess;
-  e = cudaFuncSetAttribute(&sat_tile_kernel_wd<TIn, TOut, A, REV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           SH::DYN_SMEM);
+  e = prepare_one_wd<TIn, TOut, A, REV, false>();
+  if (e == cudaSuccess) e = prepare_one_wd<TIn, TOut, A, REV, true>();
   if (e == cudaSuccess && dev >= 0 && dev < kMaxDev) done[dev].store(1, std::memory_order_release);
   return e;
 }
 
 template <class TIn, class TOut, class A, bool REV>
 cudaError_t launch_impl_wd(const SatParams& p, int grid, cudaStream_t s) {
-  using SH = TileShapeWD<TIn, TOut, A>;
   cudaError_t e = prepare_impl_wd<TIn, TOut, A, REV>();
   if (e != cudaSuccess) return e;
-  sat_tile_kernel_wd<TIn, TOut, A, REV><<<grid, SH::THREADS, SH::DYN_SMEM, s>>>(p);
+  using SH = TileShapeWD<TIn, TOut, A, false>;
+  using SK = TileShapeWD<TIn, TOut, A, true>;
+  if (p.skewed) sat_tile_kernel_wd<TIn, TOut, A, REV, true><<<grid, SK::THREADS, SK::DYN_SMEM, s>>>(p);
+  else sat_tile_kernel_wd<TIn, TOut, A, REV, false><<<grid, SH::THREADS, SH::DYN_SMEM, s>>>(p);
   return cudaGetLastError();
 }
 
@@ -152,12 +159,12 @@ cudaError_t launch_impl_wd(const SatParams& p, int grid, cudaStream_t s) {
 template <class TIn, class TOut, class A, bool REV>
 Variant make_variant_5(int in_t, int out_t, int mode) {
   if constexpr (sizeof(TIn) == 1 && sizeof(A) == 4) {
-    using SH = TileShapeWD<TIn, TOut, A>;
+    using SH = TileShapeWD<TIn, TOut, A, true>; // the larger one: both have one CTA an SM
     return Variant{in_t, out_t, mode, REV ? 1 : 0, 5,
                    &launch_impl_wd<TIn, TOut, A, REV>,
                    &prepare_impl_wd<TIn, TOut, A, REV>,
-                   (const void*)&sat_tile_kernel_wd<TIn, TOut, A, REV>,
-                   SH::TH, SH::TW, Ar<A>::K, SH::THREADS, SH::DYN_SMEM};
+                   (const void*)&sat_tile_kernel_wd<TIn, TOut, A, REV, true>,
+                   SH::TH, SH::TW, Ar<A>::K, SH::THREADS, SH::DYN_SMEM, SH::SKEW_W};
   } else {
     return make_variant_ws<TIn, TOut, A, REV, 8, sizeof(A) == 8 ? 8 : 16, true>(in_t, out_t, mode, 5);
   }

@@ -80,13 +80,16 @@ struct ImageDesc {
   // map ([tma_*_w, width)) are loaded and stored with plain accesses.
   int64_t tma_in_w, tma_out_w;
   int32_t ntx, nty;  // tiles across / down (per plane)
-  uint32_t flags;    // kInVec | kOutVec | kInTma | kOutTma
-  uint32_t pad;
+  uint32_t flags;    // kInVec | kOutVec | kInTma | kOutTma | kInSkew
+  uint32_t skew;     // kInSkew: log2 of the rows a row of tmap_in holds
 };
 constexpr uint32_t kInVec = 1u;  // every thread's CPT-element input row segment is vector-aligned
 constexpr uint32_t kOutVec = 2u; // every 16-byte output row segment is aligned
 constexpr uint32_t kInTma = 4u;  // tmap_in is valid: tiles arrive by TMA
 constexpr uint32_t kOutTma = 8u; // tmap_out is valid: results leave by TMA
+// tmap_in views 2^skew packed rows, whose bytes are a multiple of 16, as one (skew_map): tiles arrive in
+// that many TMA loads, rows off 16-byte boundaries.  Kernels of variants with skew_w only.
+constexpr uint32_t kInSkew = 16u;
 
 struct SatParams {
   ImageDesc img0;          // the image when n_images == 1
@@ -103,6 +106,7 @@ struct SatParams {
   // order whose every tile comes after the tiles it depends on (nullptr: the
   // images one after the other, each in the kernel's own order).
   const ulonglong2* order;
+  int skewed; // an image of the launch has kInSkew
 };
 
 // Pipeline depth.  A stage holds one tile from its TMA load until its TMA
@@ -606,7 +610,7 @@ struct ImageView {
   void* out;
   int64_t in_pitch, out_pitch, width, height, in_plane, out_plane, tma_in_w, tma_out_w;
   int32_t ntx, nty;
-  uint32_t flags;
+  uint32_t flags, skew;
 };
 
 __device__ __forceinline__ ImageView image_view(const SatParams& P, int img) {
@@ -625,6 +629,7 @@ __device__ __forceinline__ ImageView image_view(const SatParams& P, int img) {
     v.ntx = P.img0.ntx;
     v.nty = P.img0.nty;
     v.flags = P.img0.flags;
+    v.skew = P.img0.skew;
   } else {
     const ImageDesc* D = &P.images[img];
     v.in = D->in;
@@ -640,6 +645,7 @@ __device__ __forceinline__ ImageView image_view(const SatParams& P, int img) {
     v.ntx = D->ntx;
     v.nty = D->nty;
     v.flags = D->flags;
+    v.skew = D->skew;
   }
   return v;
 }

@@ -48,17 +48,56 @@ struct WordWait {
   }
 };
 
-template <class TIn, class TOut, class A>
+// SKEW: images whose packed rows are off 16-byte boundaries come through a map of row groups (kInSkew), with
+// others beside them; the launches of aligned images alone leave that out (with it they took 3 to 6 % more).
+template <class TIn, class TOut, class A, bool SKEW>
 struct TileShapeWD {
   static constexpr int CPT = 4, RPW = 8, NWC = 16;
   static constexpr int TW = 128, TH = NWC * RPW;
   static constexpr int NPW = TW / 32, NVW = 4, NRW = TH / 32; // summing, resolving warps (and of them, with rows)
-  static constexpr int STAGE_BYTES = TH * TW;
+  // Rows off 16-byte boundaries come with the 16 bytes that cover their shift.
+  static constexpr int SKEW_W = TW + 16;
+  static constexpr int STAGE_BYTES = TH * (SKEW ? SKEW_W : TW);
   static constexpr int STATIC_BYTES = (kWdDepth * (NWC * TW + TH + 2 * TW + TH + NWC + NRW + 4)) * 4 + 512;
   static constexpr int S = Stages<STAGE_BYTES, STATIC_BYTES, 1>::value;
   static constexpr int DYN_SMEM = S * STAGE_BYTES;
   static constexpr int THREADS = (NWC + NPW + NVW + 2) * 32;
 };
+
+// Sends tile `tp` of an image whose packed rows are off 16-byte boundaries to stage `st`, in the
+// 2^skew loads of its tensor map: rows r, r + 2^skew, ... of the tile share their shift and are one box, each
+// box's rows after the last box's, from the 16-byte boundary at or before their first pixel.
+template <class SH, class TIn>
+__device__ __forceinline__ void issue_skewed(const ImageDesc* D, const TilePlan& tp, TIn* stage, uint32_t bar) {
+  mbar_arrive_expect_tx(bar, (uint32_t)SH::STAGE_BYTES);
+  const int n = (int)D->skew, boxes = 1 << n;
+  const int pitch = (int)D->in_pitch, y = (tp.ty * SH::TH) >> n;
+  for (int q = 0; q < boxes; ++q)
+    tma_load_3d(smem_u32(stage) + q * ((SH::TH >> n) * SH::SKEW_W), &D->tmap_in, (q * pitch + tp.tx * SH::TW) & ~15, y, 0,
+                bar);
+}
+// where row `row` of such a tile starts in its stage
+template <class SH>
+__device__ __forceinline__ uint32_t skewed_row(const ImageView& D, int row) {
+  const int q = row & ((1 << D.skew) - 1);
+  return (uint32_t)(q * ((SH::TH >> D.skew) * SH::SKEW_W) + (row >> D.skew) * SH::SKEW_W + ((q * (int)D.in_pitch) & 15));
+}
+// A warp's rows of such a tile, N = its skew: the words of the lane's four pixels, from the two aligned words that
+// hold them.  (`pitch` in bytes: rows r, r + 2^N have the same shift.)
+template <class SH, int N>
+__device__ __forceinline__ void skewed_words(const void* stage, int warp, int lane, uint32_t pitch,
+                                             uint32_t (&w)[SH::RPW]) {
+  constexpr int BOX = (SH::TH >> N) * SH::SKEW_W, R = 1 << N;
+  const int q0 = (warp * SH::RPW) & (R - 1);
+  const char* base = static_cast<const char*>(stage) + q0 * BOX + ((warp * SH::RPW) >> N) * SH::SKEW_W + lane * 4;
+#pragma unroll
+  for (int r = 0; r < SH::RPW; ++r) {
+    const uint32_t shift = (uint32_t)(q0 + (r & (R - 1))) * pitch; // mod 16
+    const uint32_t* p =
+        reinterpret_cast<const uint32_t*>(base + (r & (R - 1)) * BOX + (r >> N) * SH::SKEW_W + (shift & 12u));
+    w[r] = __funnelshift_r(p[0], p[1], shift * 8u); // by the low five bits
+  }
+}
 
 // The sum of a word's four pixels picked by the mask's bytes (0 or 1), plus c.
 template <class TIn>
@@ -74,10 +113,10 @@ __device__ __forceinline__ A small_int(uint32_t v) {
   else return v;
 }
 
-template <class TIn, class TOut, class A, bool REV>
-__global__ void __launch_bounds__(TileShapeWD<TIn, TOut, A>::THREADS, 1)
+template <class TIn, class TOut, class A, bool REV, bool SKEW>
+__global__ void __launch_bounds__(TileShapeWD<TIn, TOut, A, SKEW>::THREADS, 1)
     sat_tile_kernel_wd(const __grid_constant__ SatParams P) {
-  using SH = TileShapeWD<TIn, TOut, A>;
+  using SH = TileShapeWD<TIn, TOut, A, SKEW>;
   constexpr int CPT = SH::CPT, RPW = SH::RPW, NWC = SH::NWC;
   constexpr int TW = SH::TW, TH = SH::TH, S = SH::S;
   constexpr int NPW = SH::NPW, NVW = SH::NVW, NRW = SH::NRW;
@@ -131,11 +170,23 @@ __global__ void __launch_bounds__(TileShapeWD<TIn, TOut, A>::THREADS, 1)
   if (warp == WSTORE && lane == 0) {
     // ---- producer thread: fills the stages, then refills each once the output phase of its
     //      tile has read it; a ticket is fetched a tile ahead ---------------------------
+    auto issue = [&](const TilePlan& tp, int st) {
+      const ImageDesc* D = (P.n_images == 1 || tp.t < 0) ? &P.img0 : &P.images[tp.img];
+      if (SKEW && tp.t >= 0 && (D->flags & kInSkew)) {
+        s_tile[st] = tp.t;
+        s_img[st] = tp.img;
+        s_tx[st] = tp.tx;
+        s_ty[st] = tp.ty;
+        s_pl[st] = tp.pl;
+        issue_skewed<SH>(D, tp, stages + st * SH::STAGE_BYTES, smem_u32(&s_full[st]));
+      } else {
+        issue_tile<TIn, TW, TH, TH * TW>(P, tp, st, stages + st * SH::STAGE_BYTES, s_tile, s_img, s_tx, s_ty, s_pl, s_full);
+      }
+    };
     bool producing = true;
     for (int s = 0; s < S && producing; ++s) {
       const TilePlan tp = plan_tile<REV>(P, atomicAdd(&P.ws->ticket, 1ull));
-      issue_tile<TIn, TW, TH, SH::STAGE_BYTES>(P, tp, s, stages + s * SH::STAGE_BYTES, s_tile, s_img, s_tx, s_ty, s_pl,
-                                              s_full);
+      issue(tp, s);
       producing = tp.t >= 0;
     }
     unsigned long long pending = producing ? atomicAdd(&P.ws->ticket, 1ull) : 0ull;
@@ -144,14 +195,34 @@ __global__ void __launch_bounds__(TileShapeWD<TIn, TOut, A>::THREADS, 1)
       if (next.t >= 0) pending = atomicAdd(&P.ws->ticket, 1ull);
       const int st = k % S;
       mbar_wait_bounded(smem_u32(&s_done[st]), (k / S) & 1, P, -1);
-      issue_tile<TIn, TW, TH, SH::STAGE_BYTES>(P, next, st, stages + st * SH::STAGE_BYTES, s_tile, s_img, s_tx, s_ty,
-                                              s_pl, s_full);
+      issue(next, st);
       producing = next.t >= 0;
     }
   }
 
   if (warp < NWC) {
     // ---- compute warps ----------------------------------------------------------
+    // The warp's rows of a tile, a word of four pixels a lane.
+    auto rows_in = [&](const ImageView& D, const TIn* stage, int nvalid, uint32_t (&w)[RPW]) {
+      if (!SKEW || !(D.flags & kInSkew)) {
+        const TIn* sb = stage + (warp * RPW) * TW + lane * CPT;
+#pragma unroll
+        for (int r = 0; r < RPW; ++r) w[r] = *reinterpret_cast<const uint32_t*>(sb + r * TW);
+        return;
+      }
+      const uint32_t pitch = (uint32_t)D.in_pitch;
+      switch (D.skew) {
+        case 1: skewed_words<SH, 1>(stage, warp, lane, pitch, w); break;
+        case 2: skewed_words<SH, 2>(stage, warp, lane, pitch, w); break;
+        case 3: skewed_words<SH, 3>(stage, warp, lane, pitch, w); break;
+        default: skewed_words<SH, 4>(stage, warp, lane, pitch, w); break;
+      }
+      // past the image's right edge the stage has the next rows' pixels
+      const uint32_t keep = nvalid >= CPT ? 0xffffffffu : (1u << (8 * nvalid)) - 1u;
+#pragma unroll
+      for (int r = 0; r < RPW; ++r) w[r] &= keep;
+    };
+
     // The sums of tile kk: false when the tickets ran out (the summing warps still get their
     // AGG arrival, to see the end).
     auto sums = [&](int kk) -> bool {
@@ -164,9 +235,25 @@ __global__ void __launch_bounds__(TileShapeWD<TIn, TOut, A>::THREADS, 1)
         const long long xt = x0 + (long long)lane * CPT;
         const long long rem = D.width - xt;
         const int nvalid = rem <= 0 ? 0 : (rem >= CPT ? CPT : (int)rem);
-        TIn* sb = stages + st * SH::STAGE_BYTES + (warp * RPW) * TW + lane * CPT;
+        TIn* stage = stages + st * SH::STAGE_BYTES;
+        TIn* sb = stage + (warp * RPW) * TW + lane * CPT;
         const bool tma = D.flags & kInTma;
-        if (!tma || (nvalid > 0 && xt + nvalid > D.tma_in_w)) {
+        if (SKEW && (D.flags & kInSkew)) {
+          // the rows after the last whole row of the map (they arrived as zeros)
+          const long long mapped = (D.height >> D.skew) << D.skew;
+          if (y0 + (warp + 1) * RPW > mapped && y0 + warp * RPW < D.height) {
+            for (int r = 0; r < RPW; ++r) {
+              const long long y = y0 + warp * RPW + r;
+              if (y < mapped || y >= D.height) continue;
+              TIn* at = stage + skewed_row<SH>(D, warp * RPW + r) + lane * CPT;
+#pragma unroll
+              for (int c = 0; c < CPT; ++c)
+                if (c < nvalid) at[c] = static_cast<const TIn*>(D.in)[y * D.in_pitch + xt + c];
+            }
+            __syncwarp();
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); // before TMA refills the stage
+          }
+        } else if (!tma || (nvalid > 0 && xt + nvalid > D.tma_in_w)) {
           // no TMA for this image, or columns past the map (they arrived as zeros)
           const TIn* gin = static_cast<const TIn*>(D.in) + (long long)s_pl[st] * D.in_plane +
                            (y0 + warp * RPW) * D.in_pitch + xt;
@@ -176,12 +263,13 @@ __global__ void __launch_bounds__(TileShapeWD<TIn, TOut, A>::THREADS, 1)
                                         c0, (D.flags & kInVec) != 0);
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); // before TMA refills the stage
         }
+        uint32_t in[RPW];
+        rows_in(D, stage, nvalid, in);
         uint32_t even = 0, odd = 0; // columns 0, 2 and 1, 3 over the rows, 16 bits each
         uint32_t t[RPW / 2];        // the lane's row totals, rows 2i and 2i + 1
 #pragma unroll
         for (int r = 0; r < RPW; ++r) {
-          const uint32_t w = *reinterpret_cast<const uint32_t*>(sb + r * TW);
-          const uint32_t b = SIGNED ? w ^ 0x80808080u : w;
+          const uint32_t b = SIGNED ? in[r] ^ 0x80808080u : in[r];
           even += b & 0x00ff00ffu;
           odd += (b >> 8) & 0x00ff00ffu;
           const uint32_t s = __dp4a(b, 0x01010101u, 0u);
@@ -227,10 +315,8 @@ __global__ void __launch_bounds__(TileShapeWD<TIn, TOut, A>::THREADS, 1)
       const long long xt = x0 + (long long)lane * CPT;
       const long long rem = D.width - xt;
       const int nvalid = rem <= 0 ? 0 : (rem >= CPT ? CPT : (int)rem);
-      const TIn* sb = stages + st * SH::STAGE_BYTES + (warp * RPW) * TW + lane * CPT;
       uint32_t w[RPW];
-#pragma unroll
-      for (int r = 0; r < RPW; ++r) w[r] = *reinterpret_cast<const uint32_t*>(sb + r * TW);
+      rows_in(D, stages + st * SH::STAGE_BYTES, nvalid, w);
       __syncwarp();
       TOut* out = static_cast<TOut*>(D.out) + (long long)s_pl[st] * D.out_plane + (y0 + warp * RPW) * D.out_pitch + xt;
       const long long left = D.height - (y0 + warp * RPW);

@@ -25,6 +25,7 @@ struct Variant {
   PrepareFn prepare;  // sets the dynamic shared-memory limit on the current device
   const void* kernel; // for occupancy queries
   int TH, TW, K, threads, dyn_smem;
+  int skew_w = 0; // columns of a box of rows off 16-byte boundaries (0: the kernel takes no such rows through TMA)
 };
 
 // Tile configurations (rows per warp, warps per CTA).
@@ -51,5 +52,10 @@ const Variant* find_variant(int in_t, int out_t, int mode, int dir, int cfg);
 void fill_image_desc(ImageDesc& d, const Variant* v, int in_t, int out_t, const void* in, void* out,
                      int64_t in_pitch, int64_t out_pitch, int64_t width, int64_t height, int64_t tile_base,
                      int64_t planes, int64_t in_plane, int64_t out_plane);
+
+// log2 of the rows of a packed input that make a multiple of 16 bytes, where the variant's kernel reads such
+// rows through TMA; 0 where it does not, or need not.
+int skew_rows(const Variant* v, const void* in, int64_t in_pitch, int64_t width, int64_t height, int64_t planes,
+              size_t in_sz);
 
 }  // namespace satgb

@@ -99,6 +99,17 @@ bool tma_ok(const void* base, int64_t width, int64_t height, int64_t pitch, int6
 int64_t tma_columns(int64_t width, size_t sz) { return (int64_t)(((size_t)width * sz / 16) * 16 / sz); }
 }  // namespace
 
+int skew_rows(const Variant* v, const void* in, int64_t in_pitch, int64_t width, int64_t height, int64_t planes,
+              size_t in_sz) {
+  // packed rows only: a view's last row may end with the buffer, and a map row must not pass it
+  if (!v->skew_w || planes > 1 || in_pitch != width || ((uintptr_t)in % 16) != 0 || (size_t)width * in_sz < 16 ||
+      width >= (1LL << 26) || height >= (1LL << 32) || ((size_t)in_pitch * in_sz) % 16 == 0)
+    return 0;
+  int n = 1;
+  while ((((size_t)in_pitch * in_sz) << n) % 16 != 0) ++n;
+  return (height >> n) > 0 ? n : 0;
+}
+
 void fill_image_desc(ImageDesc& d, const Variant* v, int in_t, int out_t, const void* in, void* out,
                      int64_t in_pitch, int64_t out_pitch, int64_t width, int64_t height, int64_t tile_base,
                      int64_t planes, int64_t in_plane, int64_t out_plane) {
@@ -138,6 +149,14 @@ void fill_image_desc(ImageDesc& d, const Variant* v, int in_t, int out_t, const 
   if (tma_ok(in, width, height, in_pitch, planes, in_plane, in_sz) &&
       encode_map(&d.tmap_in, in_t, in, d.tma_in_w, height, in_pitch, planes, in_plane, v->TW, v->TH))
     flags |= kInTma;
+  if (const int n = (flags & kInTma) ? 0 : skew_rows(v, in, in_pitch, width, height, planes, in_sz)) {
+    // the whole groups of 2^n rows; the kernel reads the rows after them with plain loads
+    const int64_t row = in_pitch << n;
+    if (encode_map(&d.tmap_in, in_t, in, row, height >> n, row, 1, row * (height >> n), v->skew_w, v->TH >> n)) {
+      flags |= kInSkew;
+      d.skew = (uint32_t)n;
+    }
+  }
   if (tma_ok(out, width, height, out_pitch, planes, out_plane, out_sz) &&
       encode_map(&d.tmap_out, out_t, out, d.tma_out_w, height, out_pitch, planes, out_plane, v->TW, v->TH))
     flags |= kOutTma;
@@ -572,7 +591,7 @@ int choose_config_locked(int in_t, int out_t, int mode, int dir, long long w, lo
 
 satgb_status launch_locked(const Variant* v, const ImageDesc* table_dev, const ImageDesc& img0,
                            long long n_images, long long n_tiles, Workspace& ws, int dev,
-                           cudaStream_t s, const ulonglong2* order = nullptr) {
+                           cudaStream_t s, const ulonglong2* order = nullptr, bool skewed = false) {
   const Layout L = layout_for(n_tiles, v);
   satgb_status st = ensure_ws(ws, L.total, s);
   if (st != SATGB_OK) return st;
@@ -593,6 +612,7 @@ satgb_status launch_locked(const Variant* v, const ImageDesc* table_dev, const I
   P.wait_limit_ns = g_wait_limit_ns.load();
   P.stall_tile = g_stall_tile.load();
   P.order = order;
+  P.skewed = skewed;
 
   cudaError_t e = v->launch(P, grid, s);
   if (e != cudaSuccess) return cuda_fail(e, "kernel launch");
@@ -675,7 +695,8 @@ satgb_status sat_single(int in_t, int out_t, int mode, int dir, const void* d_in
   satgb::RepackJob job{};
   bool staged = false;
   if (planes == 1 && in_sz == 1 && width * height >= kStageMinPixels && width >= 16 &&
-      !tma_ok(d_in, width, height, in_pitch, 1, 0, in_sz)) {
+      !tma_ok(d_in, width, height, in_pitch, 1, 0, in_sz) &&
+      !skew_rows(v, d_in, in_pitch, width, height, planes, in_sz)) {
     const size_t pitch = ((size_t)width + 15) & ~(size_t)15;
     st = ensure_stage(ws, pitch * (size_t)height, s);
     if (st != SATGB_OK) return st;
@@ -713,7 +734,7 @@ satgb_status sat_single(int in_t, int out_t, int mode, int dir, const void* d_in
     st = repack_launch_one(job, height, sms_of(dev), s);
     if (st != SATGB_OK) return st;
   }
-  return launch_locked(v, nullptr, d, 1, n_tiles, ws, dev, s);
+  return launch_locked(v, nullptr, d, 1, n_tiles, ws, dev, s, nullptr, (d.flags & kInSkew) != 0);
 }
 
 }  // namespace
@@ -737,6 +758,7 @@ struct BatchSeg {
   ImageDesc img0;
   ImageDesc* table = nullptr;          // device: the descriptors, then the tile order
   ulonglong2* order = nullptr; // inside the same allocation (nullptr: images one after the other)
+  bool skewed = false;         // an image has kInSkew
 };
 
 struct satgb_batch_plan_s {
@@ -1125,13 +1147,19 @@ std::vector<ulonglong2> diagonal_order(const std::vector<ImageDesc>& table) {
   return order;
 }
 
+// The kernel of configuration `cfg` for a class (nullptr: none for its types).
+const Variant* seg_variant(const satgb_batch_plan_s* p, int cls, int cfg) {
+  const Variant* v = find_variant(p->in_t, p->out_t, p->mode, p->dir, cfg);
+  if (!v) v = find_variant(p->in_t, p->out_t, p->mode, p->dir, batch_default_config(p, cls));
+  if (!v) v = find_variant(p->in_t, p->out_t, p->mode, p->dir, 0);
+  return v;
+}
+
 // (Re)builds a class's descriptor table for the configuration `cfg`; called
 // with g_mu held.
 satgb_status seg_build(satgb_batch_plan_s* p, int cls, int cfg, cudaStream_t s) {
   BatchSeg& g = p->seg[cls];
-  const Variant* v = find_variant(p->in_t, p->out_t, p->mode, p->dir, cfg);
-  if (!v) v = find_variant(p->in_t, p->out_t, p->mode, p->dir, batch_default_config(p, cls));
-  if (!v) v = find_variant(p->in_t, p->out_t, p->mode, p->dir, 0);
+  const Variant* v = seg_variant(p, cls, cfg);
   if (!v) return fail(SATGB_ERR_UNSUPPORTED_TYPES, "no kernel for this batch");
   std::vector<ImageDesc> table;
   long long base = 0;
@@ -1144,6 +1172,7 @@ satgb_status seg_build(satgb_batch_plan_s* p, int cls, int cfg, cudaStream_t s) 
   seg_free(g);
   g.v = v;
   g.n_tiles = base;
+  g.skewed = std::any_of(table.begin(), table.end(), [](const ImageDesc& d) { return (d.flags & kInSkew) != 0; });
   if (table.empty()) return SATGB_OK;
   g.img0 = table[0];
   const std::vector<ulonglong2> order = table.size() > 1 ? diagonal_order(table) : std::vector<ulonglong2>();
@@ -1186,7 +1215,7 @@ satgb_status plan_launch_locked(satgb_batch_plan_s* p, cudaStream_t s) {
   if (st0 != SATGB_OK) return st0;
   for (auto& g : p->seg) {
     if (!g.n_tiles) continue;
-    satgb_status st = launch_locked(g.v, g.table, g.img0, g.n_images, g.n_tiles, p->ws, p->dev, s, g.order);
+    satgb_status st = launch_locked(g.v, g.table, g.img0, g.n_images, g.n_tiles, p->ws, p->dev, s, g.order, g.skewed);
     if (st != SATGB_OK) return st;
   }
   return SATGB_OK;
@@ -1231,19 +1260,26 @@ void plan_free(satgb_batch_plan_s* p) {
 }
 
 // Inputs that TMA cannot address (base or row pitch not 16-byte aligned, at
-// least 16 bytes a row) get a copy in padded rows: the plan's staging buffer,
+// least 16 bytes a row), and whose class's kernel (`vs`) does not read packed rows
+// through TMA as they are, get a copy in padded rows: the plan's staging buffer,
 // one region per image (256-byte aligned, rows of the width rounded up to 16
 // bytes), and the tile kernels read the copies.  Rewrites the images' input
-// pointers and pitches in `imgs`.
-satgb_status plan_stage_inputs(satgb_batch_plan_s* p, std::vector<ImgCheck>& imgs, size_t in_sz, cudaStream_t s) {
+// pointers and pitches.
+satgb_status plan_stage_inputs(satgb_batch_plan_s* p, const Variant* const (&vs)[kBatchClasses], size_t in_sz,
+                               cudaStream_t s) {
   std::vector<satgb::RepackJob> jobs;
-  std::vector<size_t> offs, which;
+  std::vector<size_t> offs;
+  std::vector<ImgCheck*> which;
   size_t total = 0;
   long long rows = 0;
-  for (size_t i = 0; i < imgs.size(); ++i) {
-    const ImgCheck& c = imgs[i];
+  std::vector<std::pair<ImgCheck*, const Variant*>> imgs;
+  for (int cls = 0; cls < kBatchClasses; ++cls)
+    for (ImgCheck& c : p->seg[cls].imgs) imgs.emplace_back(&c, vs[cls]);
+  for (auto& [img, v] : imgs) {
+    ImgCheck& c = *img;
     const size_t row_bytes = (size_t)c.width * in_sz;
     if (row_bytes < 16 || tma_ok(c.in, c.width, c.height, c.in_pitch, 1, 0, in_sz)) continue;
+    if (v && skew_rows(v, c.in, c.in_pitch, c.width, c.height, 1, in_sz)) continue;
     const size_t pitch = (row_bytes + 15) & ~(size_t)15;
     satgb::RepackJob j;
     j.src = static_cast<const unsigned char*>(c.in);
@@ -1253,7 +1289,7 @@ satgb_status plan_stage_inputs(satgb_batch_plan_s* p, std::vector<ImgCheck>& img
     j.row_bytes = (int64_t)row_bytes;
     j.row_base = rows;
     jobs.push_back(j);
-    which.push_back(i);
+    which.push_back(&c);
     offs.push_back(total);
     total += ((pitch * (size_t)c.height) + 255) & ~(size_t)255;
     rows += c.height;
@@ -1262,7 +1298,7 @@ satgb_status plan_stage_inputs(satgb_batch_plan_s* p, std::vector<ImgCheck>& img
   p->stage = ws_alloc(total);
   if (!p->stage) return fail(SATGB_ERR_ALLOC, "batch staging allocation of %zu bytes failed", total);
   for (size_t k = 0; k < jobs.size(); ++k) {
-    ImgCheck& c = imgs[which[k]];
+    ImgCheck& c = *which[k];
     jobs[k].dst = static_cast<unsigned char*>(p->stage) + offs[k];
     c.in = jobs[k].dst;
     c.in_pitch = jobs[k].dst_pitch / (int64_t)in_sz;
@@ -1318,11 +1354,6 @@ satgb_status satgb_batch_plan_create(satgb_batch_plan** plan, satgb_dtype in_t, 
   p->mode = mode;
   p->dir = direction;
   p->dev = dev;
-  st = plan_stage_inputs(p, keep, in_sz, s);
-  if (st != SATGB_OK) {
-    plan_free(p);
-    return st;
-  }
   const int cpt = (int)(16 / out_sz);
   for (auto& c : keep) {
     const long long tiles = ((c.width + 32LL * cpt - 1) / (32LL * cpt)) * ((c.height + 127) / 128);
@@ -1330,20 +1361,27 @@ satgb_status satgb_batch_plan_create(satgb_batch_plan** plan, satgb_dtype in_t, 
     g.imgs.push_back(c);
     g.n_images += 1;
     g.pixels += (double)c.width * (double)c.height;
-    p->all_tma = p->all_tma && ((uintptr_t)c.in % 16) == 0 && ((uintptr_t)c.out % 16) == 0 &&
-                 ((size_t)c.in_pitch * in_sz) % 16 == 0 && ((size_t)c.out_pitch * out_sz) % 16 == 0;
+    // (rows of 16 bytes and more that are not are staged, or the kernel reads them through TMA as they are)
+    p->all_tma = p->all_tma && ((uintptr_t)c.out % 16) == 0 && ((size_t)c.out_pitch * out_sz) % 16 == 0 &&
+                 ((((uintptr_t)c.in % 16) == 0 && ((size_t)c.in_pitch * in_sz) % 16 == 0) ||
+                  (size_t)c.width * in_sz >= 16);
   }
   tune_load_locked();
   const int sms = sms_of(dev);
-  for (int cls = 0; cls < kBatchClasses && st == SATGB_OK; ++cls) {
+  int cfgs[kBatchClasses] = {};
+  const Variant* vs[kBatchClasses] = {};
+  for (int cls = 0; cls < kBatchClasses; ++cls) {
     if (!p->seg[cls].n_images) continue;
-    int cfg = g_forced_config;
-    if (cfg < 0) {
+    cfgs[cls] = g_forced_config;
+    if (cfgs[cls] < 0) {
       auto it = g_batch_tune.find(batch_key(p, cls, sms));
-      cfg = it != g_batch_tune.end() ? it->second : batch_default_config(p, cls);
+      cfgs[cls] = it != g_batch_tune.end() ? it->second : batch_default_config(p, cls);
     }
-    st = seg_build(p, cls, cfg, s);
+    vs[cls] = seg_variant(p, cls, cfgs[cls]);
   }
+  st = plan_stage_inputs(p, vs, in_sz, s);
+  for (int cls = 0; cls < kBatchClasses && st == SATGB_OK; ++cls)
+    if (p->seg[cls].n_images) st = seg_build(p, cls, cfgs[cls], s);
   if (st == SATGB_OK) st = plan_ws(p, s);
   if (st == SATGB_OK && p->n_tiles > 0) st = plan_capture(p);
   if (st != SATGB_OK) {
@@ -1377,11 +1415,11 @@ satgb_status satgb_batch_plan_autotune(satgb_batch_plan* p, satgb_stream stream,
       if (st == SATGB_OK) st = plan_ws(p, s);
       if (st != SATGB_OK) break;
       for (int i = 0; i < 2 && st == SATGB_OK; ++i)
-        st = launch_locked(g.v, g.table, g.img0, g.n_images, g.n_tiles, p->ws, p->dev, s, g.order);
+        st = launch_locked(g.v, g.table, g.img0, g.n_images, g.n_tiles, p->ws, p->dev, s, g.order, g.skewed);
       const int reps = 5;
       cudaEventRecord(e0, s);
       for (int i = 0; i < reps && st == SATGB_OK; ++i)
-        st = launch_locked(g.v, g.table, g.img0, g.n_images, g.n_tiles, p->ws, p->dev, s, g.order);
+        st = launch_locked(g.v, g.table, g.img0, g.n_images, g.n_tiles, p->ws, p->dev, s, g.order, g.skewed);
       cudaEventRecord(e1, s);
       cudaError_t e = cudaEventSynchronize(e1);
       if (e != cudaSuccess) st = cuda_fail(e, "cudaEventSynchronize");

@@ -791,3 +791,40 @@ def test_packed_sums_of_one_byte_pixels(cuda, pair, pixels):
         sat_gb300.stream_check()
     finally:
         sat_gb300.set_config(-1)
+
+
+@pytest.mark.parametrize("t_in,t_out", [(torch.uint8, torch.uint32), (torch.int8, torch.int32), (torch.uint8, torch.float32)])
+def test_packed_rows_through_their_map(cuda, t_in, t_out):
+    """Packed 1-byte rows whose length is no multiple of 16 (2, 4, 8 or 16 rows make one), read through
+    a map of whole groups of rows: every remainder of the length, image heights with and without rows
+    after the last group, tile edges, one image and a plan of them, both directions, bit for bit."""
+    g = torch.Generator(device="cpu").manual_seed(17)
+    info = torch.iinfo(t_in)
+
+    def same(out, ref):
+        if t_out == torch.float32:
+            return torch.equal(out.double(), ref.double())  # sums below 2^24: exact
+        return torch.equal(out.view(torch.int32).to(torch.int64) & 0xFFFFFFFF, ref & 0xFFFFFFFF)
+
+    try:
+        sat_gb300.set_config(5)
+        for rev in (False, True):
+            ins, refs = [], []
+            for w in list(range(15, 34)) + [40, 100, 127, 129, 130, 132, 136, 255, 257, 391]:
+                for h in (1, 2, 15, 16, 17, 127, 130, 144, 151):
+                    x = torch.randint(info.min, info.max + 1, (h, w), dtype=t_in, generator=g)
+                    ref = x.to(torch.int64).flip((0, 1)) if rev else x.to(torch.int64)
+                    ref = ref.cumsum(0).cumsum(1)
+                    ins.append(x.to(cuda))
+                    refs.append((ref.flip((0, 1)) if rev else ref).to(cuda))
+            for x, ref in zip(ins, refs):
+                assert same(sat_gb300.sat(x, t_out, reverse=rev), ref), (tuple(x.shape), rev)
+            outs = [torch.empty(x.shape, dtype=t_out, device=cuda) for x in ins]
+            plan = sat_gb300.BatchPlan(ins, outs, reverse=rev)
+            plan.exec()
+            plan.check()
+            for x, out, ref in zip(ins, outs, refs):
+                assert same(out, ref), (tuple(x.shape), rev)
+            plan.close()
+    finally:
+        sat_gb300.set_config(-1)
