@@ -158,7 +158,7 @@ cudaError_t launch_impl_wd(const SatParams& p, int grid, cudaStream_t s) {
 // stores for every other accumulator.
 template <class TIn, class TOut, class A, bool REV>
 Variant make_variant_5(int in_t, int out_t, int mode) {
-  if constexpr (sizeof(TIn) == 1 && sizeof(A) == 4) {
+  if constexpr (sizeof(TIn) <= 4 && sizeof(A) == 4) {
     using SH = TileShapeWD<TIn, TOut, A, true>; // the larger one: both have one CTA an SM
     return Variant{in_t, out_t, mode, REV ? 1 : 0, 5,
                    &launch_impl_wd<TIn, TOut, A, REV>,

@@ -263,7 +263,7 @@ Layout layout_for(long long n_tiles, const Variant* v) {
   L.row_off = sizeof(WsHeader);
   L.col_off = L.row_off + (size_t)n_tiles * v->TH * v->K * w;
   L.corner_off = L.col_off + (size_t)n_tiles * v->TW * v->K * w;
-  L.total = L.corner_off + (size_t)n_tiles * v->K * w;
+  L.total = L.corner_off + (size_t)n_tiles * std::max(v->K, 2) * w; // (configuration 5 keeps f32 corners in f64)
   return L;
 }
 
@@ -535,10 +535,10 @@ int sms_of(int dev) {
 
 // Heuristic default when no tuning entry exists, from measurements on GB300
 // (CUDA events, square images 1024^2 .. 32768^2):
-// 4-byte accumulators: the warp-specialized direct-store tiles (configuration
-// 5) once there are at least 4 tiles of 128 x 128 per SM (f32: 2959 vs 2851
-// GB/s at 4096^2, 4521 vs 3893 at 8192^2, 5510 vs 4370 at 16384^2), else the
-// 128-row pipelined tiles (1494 vs 1369 GB/s at 2048^2).
+// 4-byte inputs and sums: configuration 5 from 3 tiles of 128 x 128 per SM of one
+// plane (us: f32 3072^2 24.1, the row-major kernel 24.4, packed 2999 x 3001 28.0 and 34.5; 4096^2
+// 39.6 and 46.4, the 128-row pipelined tiles 45.5; 8192^2 113.5, 232, 125; i32 3072^2 23.7, 26.8,
+// 26.5), below that the row-major kernel (f32 2048^2 14.9, configuration 5 17.4).
 // 1-byte inputs with 4-byte sums: the packed kernel of configuration 5 from 3
 // tiles per SM of one plane (u8 -> u32, us: 3072^2 20.8, the row-major kernel
 // 22.5 and the 256-row direct-store tiles 24.7; 4096^2 27.6, 36.0, 33.0; 8192^2
@@ -574,7 +574,7 @@ int default_config(long long width, long long height, int sms, int in_sz, int ou
     if (ntx * ((height + 255) / 256) * std::max(1LL, planes) >= 64) return 4;
     return 1;
   }
-  if (plane_tiles >= 4LL * sms) return 5;
+  if (plane_tiles >= 3LL * sms) return 5;
   return single ? 6 : 1;
 }
 

@@ -184,7 +184,6 @@ extern "C" satgb_status satgb_sat_noalloc(const satgb_sat_desc* d, satgb_stream 
   P.col_words = (unsigned long long*)(b + col_off);
   P.corner_words = (unsigned long long*)(b + corner_off);
   P.wait_limit_ns = 2000000000LL;
-  P.skewed = (img.flags & kInSkew) != 0;
   P.stall_tile = -1;
   e = v->launch(P, grid, s);
   if (e != cudaSuccess) return noalloc_fail(SATGB_ERR_CUDA, std::string("kernel launch: ") + cudaGetErrorString(e));

@@ -828,3 +828,40 @@ def test_packed_rows_through_their_map(cuda, t_in, t_out):
             plan.close()
     finally:
         sat_gb300.set_config(-1)
+
+
+@pytest.mark.parametrize("cfg", [5, -1])
+@pytest.mark.parametrize("t", [torch.int32, torch.float32, torch.uint32])
+def test_packed_rows_of_4_bytes(cuda, t, cfg):
+    """Packed 4-byte rows off 16-byte boundaries (2 or 4 of them make a multiple): every remainder of
+    the width, heights with and without rows after the last group, tile edges, images of many tiles,
+    in place and out of place, one image and a plan, both directions.  Sums stay below 2^24: f32 is exact."""
+    g = torch.Generator(device="cpu").manual_seed(23)
+    bits = torch.int32 if t == torch.uint32 else t
+    try:
+        sat_gb300.set_config(cfg)
+        for rev in (False, True):
+            ins, refs = [], []
+            for h, w in [(h, w) for w in (4, 5, 6, 7, 9, 127, 129, 130, 131, 133, 257, 390) for h in (1, 2, 3, 4, 95, 97, 130)] + \
+                        [(1203, 1999), (2002, 1001), (700, 6001)]:
+                x = torch.randint(0, 5, (h, w), generator=g).to(bits)
+                ref = x.to(torch.int64).flip((0, 1)) if rev else x.to(torch.int64)
+                ref = ref.cumsum(0).cumsum(1)
+                ins.append(x.to(cuda))
+                refs.append((ref.flip((0, 1)) if rev else ref).to(bits).to(cuda))
+            for x, ref in zip(ins, refs):
+                out = sat_gb300.sat(x.view(t), t, reverse=rev)
+                assert torch.equal(out.view(bits), ref), (tuple(x.shape), rev)
+                y = x.clone()
+                sat_gb300.sat(y.view(t), t, reverse=rev, out=y.view(t))
+                assert torch.equal(y, ref), (tuple(x.shape), rev, "in place")
+            outs = [torch.empty_like(x) for x in ins]
+            plan = sat_gb300.BatchPlan([x.view(t) for x in ins], [o.view(t) for o in outs], reverse=rev)
+            plan.exec()
+            plan.check()
+            for out, ref in zip(outs, refs):
+                assert torch.equal(out, ref), (tuple(ref.shape), rev, "plan")
+            plan.close()
+        sat_gb300.stream_check()
+    finally:
+        sat_gb300.set_config(-1)
