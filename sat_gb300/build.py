@@ -30,6 +30,7 @@ SOURCES = [
     "sat_inst_f64.cu",
     "box_filter.cu",
     "scan_rows_t.cu",
+    "scan_cols.cu",
     "satgb_noalloc.cu",
     "batch_repack.cu",
 ]

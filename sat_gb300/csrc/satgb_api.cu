@@ -627,6 +627,10 @@ namespace satgb {
 satgb_status scan_rows_strips(int in_t, int out_t, const void* d_in, int64_t in_pitch, int64_t in_plane, void* d_out,
                               int64_t out_pitch, int64_t out_plane, int64_t width, int64_t height, int64_t planes,
                               cudaStream_t s);
+bool scan_cols_by_strips(const void* in, int64_t in_pitch, size_t in_sz, const void* out, int64_t out_pitch,
+                         size_t out_sz, int64_t width, int64_t height, int sms);
+satgb_status scan_cols_strips(int in_t, int out_t, const void* d_in, int64_t in_pitch, void* d_out, int64_t out_pitch,
+                              int64_t width, int64_t height, cudaStream_t s);
 }  // namespace satgb
 namespace {
 constexpr int kModeCols = 3;
@@ -674,6 +678,10 @@ satgb_status sat_single(int in_t, int out_t, int mode, int dir, const void* d_in
   int dev = 0;
   st = get_device(&dev);
   if (st != SATGB_OK) return st;
+  // ... nor has the column-only scan of wide images (scan_cols.cu)
+  if (mode == kModeCols && dir == SATGB_FORWARD && planes == 1 &&
+      scan_cols_by_strips(d_in, in_pitch, in_sz, d_out, out_pitch, out_sz, width, height, sms_of(dev)))
+    return scan_cols_strips(in_t, out_t, d_in, in_pitch, d_out, out_pitch, width, height, s);
   int cfg = force_cfg >= 0 ? force_cfg
             : (mode >= kModeRows) ? 1
                                   : choose_config_locked(in_t, out_t, mode, dir, width, height, dev, planes);

@@ -865,3 +865,55 @@ def test_packed_rows_of_4_bytes(cuda, t, cfg):
         sat_gb300.stream_check()
     finally:
         sat_gb300.set_config(-1)
+
+
+@pytest.mark.parametrize("t_in,t_out", [(torch.uint8, torch.uint32), (torch.int8, torch.float32), (torch.int32, torch.int32),
+                                        (torch.float32, torch.float32), (torch.int8, torch.float64),
+                                        (torch.float64, torch.float64)])
+def test_column_scan_by_strips_and_by_tiles(cuda, t_in, t_out):
+    """Column scans on both sides of the choice between strips of columns and tiles: strip and
+    block edges (32 columns, 256 rows), low and wide, narrow and tall, packed and padded rows, in place
+    where the types allow it.  Small integers: every type's sums are exact."""
+    g = torch.Generator(device="cpu").manual_seed(29)
+    for h, w in [(1, 1), (1, 33), (7, 31), (8, 32), (255, 33), (256, 64), (257, 31), (511, 1000), (513, 4864), (769, 4865),
+                 (1024, 1024), (3000, 37), (9000, 64), (2100, 5001), (300, 20001), (4100, 4096)]:
+        for pad in (0, 3):
+            x = torch.randint(0, 4, (h, w + pad), generator=g).to(t_in).to(cuda)[:, :w]
+            ref = x.to(torch.int64).cumsum(0)
+            bits = torch.int32 if t_out == torch.uint32 else t_out
+            out = sat_gb300.scan_cols(x, t_out).view(bits)
+            assert torch.equal(out, ref.to(bits)), (h, w, pad)
+            if t_in == t_out:
+                y = x.clone(memory_format=torch.contiguous_format)
+                sat_gb300.scan_cols(y, t_out, out=y)
+                assert torch.equal(y, ref.to(bits)), (h, w, pad, "in place")
+    sat_gb300.stream_check()
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan"), 3e38])
+def test_infinities_reach_what_their_element_reaches(cuda, value):
+    """An infinity, a NaN or sums past the largest f32 change the sums that contain them and
+    no other: the tile kernel of configuration 5 (aligned and packed rows) and column scans by strips and
+    by tiles, against torch's sums of the same f32 image in f64, rounded to f32."""
+    try:
+        for h, w in [(500, 512), (601, 389), (3000, 40)]:
+            x = torch.ones((h, w), device=cuda)
+            x[h // 2, w // 3] = value
+            x[h // 3, w // 2] = 3e38 if value == 3e38 else 1.0
+            y = x.double()
+            cols, sats = y.cumsum(0).float(), y.cumsum(0).cumsum(1).float()
+
+            def same(got, want):
+                if value == value and abs(value) != float("inf"):
+                    return torch.allclose(got, want, rtol=1e-5, atol=0)
+                return torch.equal(got.isnan(), want.isnan()) and torch.equal(got.nan_to_num(0, 0, 0) == 0,
+                                                                             want.nan_to_num(0, 0, 0) == 0)
+
+            assert same(sat_gb300.scan_cols(x, torch.float32), cols), (h, w)
+            sat_gb300.set_config(5)
+            assert same(sat_gb300.sat(x, torch.float32), sats), (h, w)
+            rev = sat_gb300.sat(x.flip((0, 1)).contiguous(), torch.float32, reverse=True).flip((0, 1))
+            assert same(rev, sats), (h, w)
+            sat_gb300.set_config(-1)
+    finally:
+        sat_gb300.set_config(-1)
