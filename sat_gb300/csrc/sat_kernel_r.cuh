@@ -164,14 +164,12 @@ __global__ void __launch_bounds__(NW * 32, MINB) sat_tile_kernel_r(const __grid_
     for (int r = 0; r < RPW; ++r) x[r].u.v = *reinterpret_cast<const typename RowSeg<TIn, CPT>::V*>(sb + r * TW);
     A colp[CPT], rowp[RPW];
 #pragma unroll
-    for (int c = 0; c < CPT; ++c) colp[c] = AR::zero();
-#pragma unroll
     for (int r = 0; r < RPW; ++r) {
-      A rs = AR::zero();
+      A rs = Cvt<A, TIn>::in(x[r].u.e[0]); // (sums start from their first term: an add to zero is an add)
 #pragma unroll
       for (int c = 0; c < CPT; ++c) {
-        colp[c] = AddIn<A, TIn>::add(colp[c], x[r].u.e[c]);
-        rs = AddIn<A, TIn>::add(rs, x[r].u.e[c]);
+        colp[c] = r ? AddIn<A, TIn>::add(colp[c], x[r].u.e[c]) : Cvt<A, TIn>::in(x[r].u.e[c]);
+        if (c) rs = AddIn<A, TIn>::add(rs, x[r].u.e[c]);
       }
       rowp[r] = rs;
     }
@@ -182,9 +180,9 @@ __global__ void __launch_bounds__(NW * 32, MINB) sat_tile_kernel_r(const __grid_
     __syncwarp();
     {
       const int r = lane / LPR, q = lane % LPR;
-      A tot = AR::zero();
+      A tot = s_tr[warp][r][(q * CH + (REV ? CH - 1 : 0)) ^ r];
 #pragma unroll
-      for (int i = 0; i < CH; ++i) tot = AR::add(tot, s_tr[warp][r][(q * CH + (REV ? CH - 1 - i : i)) ^ r]);
+      for (int i = 1; i < CH; ++i) tot = AR::add(tot, s_tr[warp][r][(q * CH + (REV ? CH - 1 - i : i)) ^ r]);
       A incl = tot;
 #pragma unroll
       for (int d = 1; d < LPR; d <<= 1) {
@@ -198,7 +196,7 @@ __global__ void __launch_bounds__(NW * 32, MINB) sat_tile_kernel_r(const __grid_
         const int idx = (q * CH + (REV ? CH - 1 - i : i)) ^ r;
         const A vv = s_tr[warp][r][idx];
         s_tr[warp][r][idx] = ex;
-        ex = AR::add(ex, vv);
+        if (i + 1 < CH) ex = AR::add(ex, vv);
       }
       if (q == (REV ? 0 : LPR - 1)) s_rowagg[warp * RPW + r] = incl;
     }
@@ -212,21 +210,21 @@ __global__ void __launch_bounds__(NW * 32, MINB) sat_tile_kernel_r(const __grid_
     // ---- look-back phase ----------------------------------------------------
     A my_agg = AR::zero();
     if (is_col) {
-      // column aggregate out at once, then the exclusive prefix over the warps
+      // the exclusive prefix over the warps, then the column aggregate
       const int j = tid;
-      A ac = AR::zero();
+      A v[NW];
 #pragma unroll
-      for (int w = 0; w < NW; ++w) ac = AR::add(ac, s_colp[w][j]);
-      if (pub_col && !stall) publish<A>(P.col_words + ((unsigned long long)t * TW + j) * K, ac, tagA);
-      A run = AR::zero();
+      for (int w = 0; w < NW; ++w) v[w] = s_colp[w][j];
+      A run = v[REV ? NW - 1 : 0];
+      s_colp[REV ? NW - 1 : 0][j] = AR::zero();
 #pragma unroll
-      for (int i = 0; i < NW; ++i) {
+      for (int i = 1; i < NW; ++i) {
         const int w = REV ? NW - 1 - i : i;
-        const A b = s_colp[w][j];
         s_colp[w][j] = run;
-        run = AR::add(run, b);
+        run = AR::add(run, v[w]);
       }
-      my_agg = ac;
+      if (pub_col && !stall) publish<A>(P.col_words + ((unsigned long long)t * TW + j) * K, run, tagA);
+      my_agg = run;
     } else if (is_row) {
       my_agg = s_rowagg[tid - TW];
       if (pub_row && !stall) publish<A>(P.row_words + ((unsigned long long)t * TH + (tid - TW)) * K, my_agg, tagA);

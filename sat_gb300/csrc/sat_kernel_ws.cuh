@@ -252,16 +252,14 @@ __global__ void __launch_bounds__(TileShapeWS<TIn, TOut, A, RPW, NWC, DIRECT, CT
       }
       A colp[CPT], rowp[RPW];
 #pragma unroll
-      for (int c = 0; c < CPT; ++c) colp[c] = AR::zero();
-#pragma unroll
       for (int r = 0; r < RPW; ++r) {
         RowSeg<TIn, CPT> x;
         x.u.v = *reinterpret_cast<const typename RowSeg<TIn, CPT>::V*>(sb + r * TW);
-        A rs = AR::zero();
+        A rs = Cvt<A, TIn>::in(x.u.e[0]); // (sums start from their first term: an add to zero is an add)
 #pragma unroll
         for (int c = 0; c < CPT; ++c) {
-          colp[c] = AddIn<A, TIn>::add(colp[c], x.u.e[c]);
-          rs = AddIn<A, TIn>::add(rs, x.u.e[c]);
+          colp[c] = r ? AddIn<A, TIn>::add(colp[c], x.u.e[c]) : Cvt<A, TIn>::in(x.u.e[c]);
+          if (c) rs = AddIn<A, TIn>::add(rs, x.u.e[c]);
         }
         rowp[r] = rs;
       }
@@ -274,9 +272,9 @@ __global__ void __launch_bounds__(TileShapeWS<TIn, TOut, A, RPW, NWC, DIRECT, CT
         __syncwarp();
         {
           const int r = lane / LPR, q = lane % LPR;
-          A tot = AR::zero();
+          A tot = s_tr[warp][r][(q * CH + (REV ? CH - 1 : 0)) ^ r];
 #pragma unroll
-          for (int i = 0; i < CH; ++i) tot = AR::add(tot, s_tr[warp][r][(q * CH + (REV ? CH - 1 - i : i)) ^ r]);
+          for (int i = 1; i < CH; ++i) tot = AR::add(tot, s_tr[warp][r][(q * CH + (REV ? CH - 1 - i : i)) ^ r]);
           A incl = tot;
 #pragma unroll
           for (int d = 1; d < LPR; d <<= 1) {
@@ -290,7 +288,7 @@ __global__ void __launch_bounds__(TileShapeWS<TIn, TOut, A, RPW, NWC, DIRECT, CT
             const int idx = (q * CH + (REV ? CH - 1 - i : i)) ^ r;
             const A vv = s_tr[warp][r][idx];
             s_tr[warp][r][idx] = ex;
-            ex = AR::add(ex, vv);
+            if (i + 1 < CH) ex = AR::add(ex, vv);
           }
           if (q == (REV ? 0 : LPR - 1)) s_rowagg[kk & 1][warp * RPW + h * RP + r] = incl;
         }
@@ -450,9 +448,10 @@ __global__ void __launch_bounds__(TileShapeWS<TIn, TOut, A, RPW, NWC, DIRECT, CT
       A v[NWC];
 #pragma unroll
       for (int w = 0; w < NWC; ++w) v[w] = s_colp[kb][w][j];
-      A run = AR::zero();
+      A run = v[REV ? NWC - 1 : 0];
+      s_colp[kb][REV ? NWC - 1 : 0][j] = AR::zero();
 #pragma unroll
-      for (int i = 0; i < NWC; ++i) {
+      for (int i = 1; i < NWC; ++i) {
         const int w = REV ? NWC - 1 - i : i;
         s_colp[kb][w][j] = run;
         run = AR::add(run, v[w]);
