@@ -750,11 +750,14 @@ satgb_status sat_single(int in_t, int out_t, int mode, int dir, const void* d_in
 // ============================================================================
 // Batch plans
 // ============================================================================
-// The images of a plan fall into two size classes, each run by its own
-// persistent launch with its own tile configuration (both launches follow one
-// another in the plan's CUDA graph, sharing one workspace): large images,
-// whose long look-back chains favour the big warp-specialized tiles, and small
-// ones, where smaller tiles or the row-major order waste less.
+// The images of a plan fall into two size classes, each with its own tile
+// configuration: large images, whose long look-back chains favour the big
+// warp-specialized tiles, and small ones, where smaller tiles or the row-major
+// order waste less.  Classes with different configurations are launches of their
+// own (following one another in the plan's CUDA graph, sharing one workspace);
+// with the same one they are one launch, so that the second's first tiles fill the SMs that
+// the first's last ones leave idle (u8 -> u32, us: 40 images of sides 64..4096 68 -> 56, in
+// 128-byte rows 72 -> 56; 512 of them 844 -> 835 and 705 -> 691).
 constexpr int kBatchClasses = 2;
 constexpr long long kLargeTiles = 64; // an image of at least 64 tiles of 128 x 128 is large
 
@@ -780,6 +783,7 @@ struct satgb_batch_plan_s {
   int n_jobs = 0;
   long long stage_rows = 0;
   BatchSeg seg[kBatchClasses];
+  BatchSeg all; // both classes' images, when they share a launch (n_tiles > 0)
   long long n_tiles = 0;
   Workspace ws;
   cudaGraph_t graph = nullptr;
@@ -1163,11 +1167,9 @@ const Variant* seg_variant(const satgb_batch_plan_s* p, int cls, int cfg) {
   return v;
 }
 
-// (Re)builds a class's descriptor table for the configuration `cfg`; called
-// with g_mu held.
-satgb_status seg_build(satgb_batch_plan_s* p, int cls, int cfg, cudaStream_t s) {
-  BatchSeg& g = p->seg[cls];
-  const Variant* v = seg_variant(p, cls, cfg);
+// (Re)builds a class's descriptor table for the kernel `v`; called with g_mu
+// held.
+satgb_status seg_build(satgb_batch_plan_s* p, BatchSeg& g, const Variant* v, cudaStream_t s) {
   if (!v) return fail(SATGB_ERR_UNSUPPORTED_TYPES, "no kernel for this batch");
   std::vector<ImageDesc> table;
   long long base = 0;
@@ -1200,8 +1202,21 @@ satgb_status seg_build(satgb_batch_plan_s* p, int cls, int cfg, cudaStream_t s) 
   return SATGB_OK;
 }
 
+// One table for both classes where they run the same kernel; called once every class has its own.
+satgb_status plan_merge(satgb_batch_plan_s* p, cudaStream_t s) {
+  seg_free(p->all);
+  p->all = BatchSeg();
+  for (auto& g : p->seg)
+    if (!g.n_tiles || g.v != p->seg[0].v) return SATGB_OK;
+  for (auto& g : p->seg) {
+    p->all.imgs.insert(p->all.imgs.end(), g.imgs.begin(), g.imgs.end());
+    p->all.n_images += g.n_images;
+  }
+  return seg_build(p, p->all, p->seg[0].v, s);
+}
+
 satgb_status plan_ws(satgb_batch_plan_s* p, cudaStream_t s) {
-  size_t need = 0;
+  size_t need = p->all.n_tiles ? layout_for(p->all.n_tiles, p->all.v).total : 0;
   p->n_tiles = 0;
   for (auto& g : p->seg)
     if (g.n_tiles) {
@@ -1218,12 +1233,22 @@ satgb_status plan_repack(satgb_batch_plan_s* p, cudaStream_t s) {
   return repack_launch(p->jobs, p->n_jobs, p->stage_rows, sms_of(p->dev), s);
 }
 
+// What a plan launches: both classes at once, or one after the other.
+std::vector<const BatchSeg*> plan_launches(const satgb_batch_plan_s* p) {
+  std::vector<const BatchSeg*> v;
+  if (p->all.n_tiles) v.push_back(&p->all);
+  else
+    for (const auto& g : p->seg)
+      if (g.n_tiles) v.push_back(&g);
+  return v;
+}
+
 satgb_status plan_launch_locked(satgb_batch_plan_s* p, cudaStream_t s) {
   satgb_status st0 = plan_repack(p, s);
   if (st0 != SATGB_OK) return st0;
-  for (auto& g : p->seg) {
-    if (!g.n_tiles) continue;
-    satgb_status st = launch_locked(g.v, g.table, g.img0, g.n_images, g.n_tiles, p->ws, p->dev, s, g.order, g.skewed);
+  for (const BatchSeg* g : plan_launches(p)) {
+    satgb_status st =
+        launch_locked(g->v, g->table, g->img0, g->n_images, g->n_tiles, p->ws, p->dev, s, g->order, g->skewed);
     if (st != SATGB_OK) return st;
   }
   return SATGB_OK;
@@ -1264,6 +1289,7 @@ void plan_free(satgb_batch_plan_s* p) {
   ws_free(p->stage);
   if (p->jobs) cudaFree(p->jobs);
   for (auto& g : p->seg) seg_free(g);
+  seg_free(p->all);
   delete p;
 }
 
@@ -1389,7 +1415,8 @@ satgb_status satgb_batch_plan_create(satgb_batch_plan** plan, satgb_dtype in_t, 
   }
   st = plan_stage_inputs(p, vs, in_sz, s);
   for (int cls = 0; cls < kBatchClasses && st == SATGB_OK; ++cls)
-    if (p->seg[cls].n_images) st = seg_build(p, cls, cfgs[cls], s);
+    if (p->seg[cls].n_images) st = seg_build(p, p->seg[cls], vs[cls], s);
+  if (st == SATGB_OK) st = plan_merge(p, s);
   if (st == SATGB_OK) st = plan_ws(p, s);
   if (st == SATGB_OK && p->n_tiles > 0) st = plan_capture(p);
   if (st != SATGB_OK) {
@@ -1419,7 +1446,7 @@ satgb_status satgb_batch_plan_autotune(satgb_batch_plan* p, satgb_stream stream,
     for (int cfg = 0; cfg < kNumConfigs && st == SATGB_OK; ++cfg) {
       const Variant* v = find_variant(p->in_t, p->out_t, p->mode, p->dir, cfg);
       if (!v || v->cfg != cfg) continue;
-      st = seg_build(p, cls, cfg, s);
+      st = seg_build(p, g, v, s);
       if (st == SATGB_OK) st = plan_ws(p, s);
       if (st != SATGB_OK) break;
       for (int i = 0; i < 2 && st == SATGB_OK; ++i)
@@ -1439,12 +1466,13 @@ satgb_status satgb_batch_plan_autotune(satgb_batch_plan* p, satgb_stream stream,
       }
     }
     if (st != SATGB_OK) break;
-    st = seg_build(p, cls, best, s);
+    st = seg_build(p, g, seg_variant(p, cls, best), s);
     g_batch_tune[batch_key(p, cls, sms)] = best;
     if (configs) configs[cls] = best;
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
+  if (st == SATGB_OK) st = plan_merge(p, s);
   if (st == SATGB_OK) st = plan_ws(p, s);
   if (st == SATGB_OK) {
     WsHeader h;
@@ -1462,8 +1490,7 @@ satgb_status satgb_batch_plan_exec(satgb_batch_plan* p, satgb_stream stream) {
   if (p->n_tiles == 0) return SATGB_OK;
   cudaError_t e = cudaGraphLaunch(p->exec, (cudaStream_t)stream);
   if (e != cudaSuccess) return cuda_fail(e, "cudaGraphLaunch");
-  for (auto& g : p->seg)
-    if (g.n_tiles) g_launches.fetch_add(1);
+  g_launches.fetch_add((long long)plan_launches(p).size());
   return SATGB_OK;
 }
 
