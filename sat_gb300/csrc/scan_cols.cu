@@ -5,15 +5,16 @@
 // the last and no sum ever crosses CTAs: no status words, no look-back, no order of tiles.  Blocks of NW x R
 // rows go through registers: a warp sums its R rows (a lane a column, rows of the strip 32 coalesced
 // elements at any alignment), the warps' sums meet in shared memory, and each warp runs down its rows from the
-// sum of everything above.  The next two blocks' loads are in flight meanwhile.
+// sum of everything above.  The next block's loads are in flight meanwhile (two blocks ahead f32 4096^2 was 26.6 us
+// for 28.5, but 4600 x 3000 30.3 for 25.9: 64 registers a thread are short).
 //
 // What bounds it: a block's time on one SM, whose stores (25 bytes a cycle at most) and whose
 // scan over the warps follow one another (1.35 us a block of 256 rows of 4-byte results, half of it the
 // stores); f64 results the FP64 adds, 7 us.  Memory only where every SM has a strip.  With 16 warps of 16
 // rows and each warp adding up the ones before it a block took 2 us, and f32 errors doubled; an f32
 // column's sum over the blocks is a two-sum pair (mean relative error at 8192 rows 7.9e-8 -> 4.6e-8).
-// us, before (look-back over tiles) and now: f32 256 x 256 7.9 -> 3.8, 1024^2 10.4 -> 8.1, 4096 x 1000 13.3 -> 8.7,
-// 4096^2 33.8 -> 27.6, packed 3001 x 3000 32.8 -> 28.7, packed 8191^2 221 -> 159; f64 4096^2 176 -> 120.
+// us, before (look-back over tiles) and now: f32 256 x 256 7.9 -> 3.4, 1024^2 10.4 -> 7.1, 4096 x 1000 13.3 -> 8.3,
+// 4096^2 33.8 -> 29, packed 3001 x 3000 32.8 -> 25.1, packed 8191^2 221 -> 146; f64 4096^2 176 -> 117.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -42,11 +43,14 @@ struct Carry {
 template <>
 struct Carry<float> {
   float s = 0.f, e = 0.f;
-  __device__ __forceinline__ float below(float x) const { return s + (e + x); }
+  __device__ __forceinline__ float below(float x) const {
+    const float y = e + x;
+    return s + (y == y ? y : x); // past the finite numbers the error term is a NaN, the sum need not be
+  }
   __device__ __forceinline__ void add(float x) {
     float err;
     s = two_sum(s, x, err);
-    e = fabsf(s) <= 3.402823466e38f ? e + err : 0.f; // past the finite numbers there is no error term
+    e += err;
   }
 };
 
@@ -113,18 +117,14 @@ __global__ void __launch_bounds__(kColWarps * 32, 1)
     gout += BLOCK * out_pitch;
   };
 
-  TIn v0[R], v1[R], v2[R];
+  TIn v0[R], v1[R];
   load(v0, 0);
-  load(v1, 1);
-  for (long long b = 0; b < n_blocks; b += 3) {
-    load(v2, b + 2);
+  for (long long b = 0; b < n_blocks; b += 2) {
+    load(v1, b + 1);
     step(v0, b);
     if (b + 1 >= n_blocks) break;
-    load(v0, b + 3);
+    load(v0, b + 2);
     step(v1, b + 1);
-    if (b + 2 >= n_blocks) break;
-    load(v1, b + 4);
-    step(v2, b + 2);
   }
 }
 
@@ -142,7 +142,7 @@ cudaError_t launch_cols(const void* in, int64_t in_pitch, void* out, int64_t out
 // faster.  Strips: 3 us and 1.4 a block of a strip (f64 results 7) for each wave of strips over the SMs, a third more
 // where rows are off 16-byte boundaries, and no faster than 4.7 TB/s.  Tiles: 8 us and 5.3 TB/s (f64 10 us and
 // 1.6), 3.0 where rows cannot go through TMA.  Few strips or many rows are the tiles': f32 1024 x 8192 (w x h)
-// 19 us by tiles, 46 by strips, 8192^2 100 and 116; wide and low, or packed, the strips': 8192 x 300 11.5 and 10.
+// 19 us by tiles, 46 by strips, 8192^2 100 and 116; wide and low, or packed, the strips': 8192 x 300 11.5 and 9.1.
 bool scan_cols_by_strips(const void* in, int64_t in_pitch, size_t in_sz, const void* out, int64_t out_pitch,
                          size_t out_sz, int64_t width, int64_t height, int sms) {
   const int64_t strips = (width + 31) / 32;
