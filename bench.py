@@ -326,9 +326,9 @@ def run_gpu(args):
         "warmup_launches": int(warm_launches),
         "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                      "frac": round(achieved / peak, 4), "peak_kind": peak_kind,
-                     "traffic": _traffic_from_profiles("f32_f32_8192_ws"),
+                     "traffic": _traffic_from_profiles("f32_f32_8192_wd"),
                      "algorithmic_bytes_per_launch": step_bytes,
-                     "kernel": "satgb::sat_tile_kernel_ws<float,float,float,fwd> (128-row tiles, direct stores)"},
+                     "kernel": "satgb::sat_tile_kernel_wd<float,float,float,fwd,aligned> (96-row tiles, direct stores)"},
         "cpu_baseline": cpu,
         "clocks": clocks,
         "sub_results": sub,

@@ -240,11 +240,13 @@ satgb_status satgb_sat_noalloc(const satgb_sat_desc* desc, satgb_stream stream);
 /* into two size classes (large: at least 64 tiles of 128 x 128 pixels;       */
 /* small: the rest), picks a tile configuration per class (from the tuning    */
 /* cache when an entry for this batch's signature exists) and captures the    */
-/* classes' launches, one after the other, in one CUDA graph; exec replays    */
+/* classes' launches, one after the other, or one launch of both where they   */
+/* take the same kernel, in one CUDA graph; exec replays                      */
 /* the graph on `stream`.  All images share one dtype pair, mode and          */
 /* direction.  No image may write memory another image reads or writes.       */
 /* Inputs whose rows TMA cannot address (base or row pitch not a multiple of  */
-/* 16 bytes, rows of at least 16 bytes: e.g. packed u8 rows of odd widths)    */
+/* 16 bytes, rows of at least 16 bytes: e.g. views and offset bases; packed   */
+/* rows too, unless the class's kernel reads them in groups)                  */
 /* are copied by each exec, as the graph's first launch, into rows padded to  */
 /* 16 bytes in a staging buffer the plan allocates (about the size of those   */
 /* inputs, through the allocator hooks when set) and frees on destroy.        */

@@ -3,11 +3,12 @@
 // A tensor map needs a 16-byte aligned base and a row pitch of whole 16-byte
 // chunks.  Images packed row after row (a pitch of width elements, e.g. u8
 // images of odd widths) have neither, and the tile kernels would read them
-// with plain loads on their compute warps.  A batch plan instead copies such
+// with plain loads on their compute warps.  Where the kernel does not read packed
+// rows through a map of row groups (sat_kernel_wd.cuh), a batch plan instead copies such
 // inputs, at each execution and inside the same graph, into rows padded to 16
 // bytes in a staging buffer of its own, and runs the tile kernels on the
 // copies through TMA; a single large image with 1-byte inputs is staged the
-// same way in its call's workspace (repack_launch_one).
+// same way in a buffer beside its call's workspace (repack_launch_one).
 //
 // One warp per row, rows of all the staged images in one launch (a job per
 // image, found by binary search over the jobs' first rows).  A lane writes
