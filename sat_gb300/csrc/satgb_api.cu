@@ -535,8 +535,11 @@ int sms_of(int dev) {
 
 // Heuristic default when no tuning entry exists, from measurements on GB300
 // (CUDA events, square images 1024^2 .. 32768^2):
-// 4-byte inputs and sums: configuration 5 from 3 tiles of 128 x 128 per SM of one
-// plane (us: f32 3072^2 24.1, the row-major kernel 24.4, packed 2999 x 3001 28.0 and 34.5; 4096^2
+// 4-byte inputs and sums: configuration 5 from 4 tiles of 128 x 128 per SM of one
+// plane, from 3 where the image is not narrow (below 16 tiles a row the row-major kernel's sums over the
+// tiles to the left are few: f32 1000 x 8192 (w x h) 22.9 us, configuration 5 23.9; 8192 x 1000
+// 27.4 and 22.4) or its packed rows are off 16-byte boundaries (1003 x 8000 31.3 and 26.5).  (us:
+// f32 3072^2 24.1, the row-major kernel 24.4, packed 2999 x 3001 28.0 and 34.5; 4096^2
 // 39.6 and 46.4, the 128-row pipelined tiles 45.5; 8192^2 113.5, 232, 125; i32 3072^2 23.7, 26.8,
 // 26.5), below that the row-major kernel (f32 2048^2 14.9, configuration 5 17.4).
 // 1-byte inputs with 4-byte sums: the packed kernel of configuration 5 from 3
@@ -548,20 +551,24 @@ int sms_of(int dev) {
 // Compensated f32: the 128-row register tiles (2474 vs 1570 GB/s for
 // configuration 5 at 8192^2, 1096 vs 911 for the 64-row tiles at 2048^2).
 // f64 outputs (slow FP64 adds on GB300): the warp-specialized tiles, whose
-// compute warps never wait at a CTA barrier.
+// compute warps never wait at a CTA barrier, from 40 tiles of 128 x 64 in one image (us,
+// them and the pipelined kernel: f64 640^2 18.3 and 20.2, 800^2 21.2 and 26.7, 1024^2 24.3 and 31.4, 2048^2
+// 70.4 and 85.5, f32 -> f64 1000 x 8192 150 and 195; 512^2 17.2 and 16.0, 256^2 15.1 and
+// 13.4); stacks of planes from 8 tiles per SM.
 // Stacks of planes count all their tiles for the size classes, but
 // configuration 5 needs its tile count in one plane: its gain is in long
 // look-back chains, and stacks of small planes (64 x 3 planes of 1024^2, the
 // box-filter layer) ran 15 % slower with it than with the pipelined tiles.
+// `off16`: packed input rows off 16-byte boundaries, which configuration 5 reads through row-group maps.
 int default_config(long long width, long long height, int sms, int in_sz, int out_sz, bool compensated,
-                   long long planes = 1) {
+                   long long planes = 1, bool off16 = false) {
   const int cpt = 16 / out_sz;
   const long long tw = 32LL * cpt;
   const long long ntx = (width + tw - 1) / tw;
   const long long plane_tiles = ntx * ((height + 127) / 128);
   const long long tiles128 = plane_tiles * std::max(1LL, planes);
   sms = std::max(1, sms);
-  if (out_sz == 8) return tiles128 >= 8LL * sms ? 0 : 2;
+  if (out_sz == 8) return tiles128 >= (planes <= 1 ? 40LL : 8LL * sms) ? 0 : 2;
   if (compensated) return tiles128 >= sms ? 3 : 2;
   // Small single images: the row-major kernel (configuration 6), whose short
   // tile rows make its sums over the row aggregates cheap (f32 1536^2 17.8 ->
@@ -574,19 +581,19 @@ int default_config(long long width, long long height, int sms, int in_sz, int ou
     if (ntx * ((height + 255) / 256) * std::max(1LL, planes) >= 64) return 4;
     return 1;
   }
-  if (plane_tiles >= 3LL * sms) return 5;
+  if (plane_tiles >= 4LL * sms || (plane_tiles >= 3LL * sms && (ntx >= 16 || off16))) return 5;
   return single ? 6 : 1;
 }
 
 int choose_config_locked(int in_t, int out_t, int mode, int dir, long long w, long long h, int dev,
-                         long long planes = 1) {
+                         long long planes = 1, bool off16 = false) {
   if (g_forced_config >= 0) return g_forced_config;
   tune_load_locked();
   const int sms = sms_of(dev);
   auto it = g_tune.find(TuneKey(in_t, out_t, mode, dir, log2_bucket(w), log2_bucket(h * std::max(1LL, planes)), sms));
   if (it != g_tune.end()) return it->second;
   return default_config(w, h, sms, (int)dtype_size(in_t), (int)dtype_size(out_t), mode == SATGB_MODE_COMPENSATED,
-                        planes);
+                        planes, off16);
 }
 
 satgb_status launch_locked(const Variant* v, const ImageDesc* table_dev, const ImageDesc& img0,
@@ -682,14 +689,15 @@ satgb_status sat_single(int in_t, int out_t, int mode, int dir, const void* d_in
   if (mode == kModeCols && dir == SATGB_FORWARD && planes == 1 &&
       scan_cols_by_strips(d_in, in_pitch, in_sz, d_out, out_pitch, out_sz, width, height, sms_of(dev)))
     return scan_cols_strips(in_t, out_t, d_in, in_pitch, d_out, out_pitch, width, height, s);
+  const bool off16 = planes == 1 && in_pitch == width && (uintptr_t)d_in % 16 == 0 && ((size_t)in_pitch * in_sz) % 16 != 0;
   int cfg = force_cfg >= 0 ? force_cfg
             : (mode >= kModeRows) ? 1
-                                  : choose_config_locked(in_t, out_t, mode, dir, width, height, dev, planes);
+                                  : choose_config_locked(in_t, out_t, mode, dir, width, height, dev, planes, off16);
   const Variant* v = find_variant(in_t, out_t, mode, dir, cfg);
   if (!v && mode < kModeRows) // a configuration this pair does not have: the untuned choice
     v = find_variant(in_t, out_t, mode, dir,
                      default_config(width, height, sms_of(dev), (int)in_sz, (int)out_sz,
-                                    mode == SATGB_MODE_COMPENSATED, planes));
+                                    mode == SATGB_MODE_COMPENSATED, planes, off16));
   if (!v) v = find_variant(in_t, out_t, mode, dir, 0);
   if (!v) return fail(SATGB_ERR_UNSUPPORTED_TYPES, "no kernel for %s -> %s mode %d dir %d", dtype_name(in_t), dtype_name(out_t), mode, dir);
   Workspace& ws = g_ws[std::make_pair(dev, (void*)s)];
