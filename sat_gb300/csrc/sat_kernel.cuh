@@ -392,18 +392,41 @@ __device__ __forceinline__ void finish_launch(const SatParams& P, uint32_t epoch
   }
 }
 
-// Bounded wait for an mbarrier phase; false (and an error recorded) when the
-// wait limit runs out.
+// A wait inside a CTA: for a copy that its producer started, a stage that its compute warps
+// have read, a value another of its warps hands over.  It ends without any other CTA: the only waits
+// for other tiles are the look-backs, and those end by themselves.  So it goes neither by the
+// wait limit nor by another CTA's error.  A role that gave up by those before its stage was first filled read tile
+// indices nobody had written, and roles that gave up at different times took different tiles from one
+// stage and no longer met at the named barriers.  What ends it when nothing else does is eight wait limits, looked at
+// every 2^24 polls, so that time in which the GPU ran something else does not count.
+struct CtaWait {
+  static constexpr uint32_t kPolls = 1u << 24;
+  uint32_t polls = 0;
+  unsigned long long t0 = 0;
+  // one more poll; false (an error recorded) when the wait has to end
+  __device__ __forceinline__ bool again(const SatParams& P, long long tile) {
+    if (t0 == 0) t0 = global_timer_ns();
+    if ((++polls & (kPolls - 1)) != 0 || (long long)((global_timer_ns() - t0) >> 3) <= P.wait_limit_ns) return true;
+    record_error(P, tile);
+    return false;
+  }
+};
+
 static __device__ __noinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity, const SatParams& P, long long tile) {
   if (mbar_try_wait(bar, parity)) return true;
-  const unsigned long long t0 = global_timer_ns();
-  for (uint32_t it = 0;; ++it) {
+  CtaWait wait;
+  while (wait.again(P, tile))
     if (mbar_try_wait(bar, parity)) return true;
-    if ((it & 63u) == 63u &&
-        ((long long)(global_timer_ns() - t0) > P.wait_limit_ns || ld_relaxed_u32(&P.ws->error) != 0u)) {
-      record_error(P, tile);
-      return false;
-    }
+  return false;
+}
+
+// Stage descriptors before the producer has written any: tile 0, which every launch has.
+template <int S>
+__device__ __forceinline__ void clear_stages(int tid, long long (&tile)[S], int (&img)[S], int (&tx)[S], int (&ty)[S],
+                                             int (&pl)[S]) {
+  if (tid < S) {
+    tile[tid] = 0;
+    img[tid] = tx[tid] = ty[tid] = pl[tid] = 0;
   }
 }
 

@@ -158,6 +158,7 @@ __global__ void __launch_bounds__(TileShapeRM<TIn, TOut, A, RPW, NWC>::THREADS, 
   const uint32_t tagI = make_tag(epoch, kStateInc);
 
   // ---- prologue: barriers; the producer fills the stages while the other roles start ------------
+  clear_stages(tid, s_tile, s_img, s_tx, s_ty, s_pl);
   if (warp == WPROD && lane == 0) {
 #pragma unroll
     for (int s = 0; s < S; ++s) {

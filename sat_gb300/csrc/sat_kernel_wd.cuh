@@ -37,21 +37,6 @@
 
 namespace satgb {
 
-// One more round of a wait; false (an error recorded) when it has to give up.
-struct WordWait {
-  uint32_t round = 0;
-  unsigned long long t0 = 0;
-  __device__ __forceinline__ bool again(const SatParams& P, long long tile) {
-    if (round == 0) t0 = global_timer_ns();
-    if ((++round & 15u) == 0u &&
-        ((long long)(global_timer_ns() - t0) > P.wait_limit_ns || ld_relaxed_u32(&P.ws->error) != 0u)) {
-      record_error(P, tile);
-      return false;
-    }
-    return true;
-  }
-};
-
 // SKEW: images whose packed rows are off 16-byte boundaries come through a map of row groups (kInSkew), with
 // others beside them; the launches of aligned images alone leave that out (with it they took 3 to 6 % more).
 template <class TIn, class TOut, class A, bool SKEW>
@@ -226,6 +211,7 @@ __global__ void __launch_bounds__(TileShapeWD<TIn, TOut, A, SKEW>::THREADS, 1)
   const uint32_t tagI = make_tag(epoch, kStateInc);
 
   if (tid < SH::D) s_uready[tid] = 0;
+  clear_stages(tid, s_tile, s_img, s_tx, s_ty, s_pl);
   if (warp == WSTORE && lane == 0) {
 #pragma unroll
     for (int s = 0; s < S; ++s) {
@@ -713,7 +699,7 @@ __global__ void __launch_bounds__(TileShapeWD<TIn, TOut, A, SKEW>::THREADS, 1)
         resolve_n<C, 1>(w, base, 0, step, ly, tagA, tagI, P, t, corner);
         // u of tile k: the resolving warps have it after every compute warp took tile k's sums, and so is done
         // with the set's last tile (nothing else keeps this warp from running ahead of them)
-        WordWait wait;
+        CtaWait wait;
         while (vload(&s_uready[kb]) != k + 1 && wait.again(P, t)) {
         }
         __threadfence_block();

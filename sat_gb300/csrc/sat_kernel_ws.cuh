@@ -132,6 +132,7 @@ __global__ void __launch_bounds__(TileShapeWS<TIn, TOut, A, RPW, NWC, DIRECT, CT
 
   // ---- prologue: barriers; the store warp fills the stages while the other roles start --------
   if (tid < 2) s_cnt_corner[tid] = 0;
+  clear_stages(tid, s_tile, s_img, s_tx, s_ty, s_pl);
   if (warp == WSTORE && lane == 0) {
 #pragma unroll
     for (int s = 0; s < S; ++s) {

@@ -917,3 +917,47 @@ def test_infinities_reach_what_their_element_reaches(cuda, value):
             sat_gb300.set_config(-1)
     finally:
         sat_gb300.set_config(-1)
+
+
+@pytest.mark.parametrize("cfg", [0, 1, 2, 3, 4, 5, 6])
+@pytest.mark.parametrize("t_in,t_out", [(torch.uint8, torch.uint32), (torch.float32, torch.float32)])
+def test_waits_that_end_early_stay_inside_the_image(cuda, cfg, t_in, t_out):
+    """With a wait limit of a microsecond and a first tile that never publishes, look-backs give up
+    everywhere while stages are still being filled for the first time: every role goes on with the
+    tiles its CTA was given, so nothing outside the result is written, the error is reported, and the next calls
+    are right.  Fewer tiles than CTAs, about as many, and many a CTA; aligned and packed rows."""
+    L = _lib.load()
+    s = torch.cuda.Stream()
+    guard = 1 << 16
+    for h, w in [(130, 260), (1500, 1601), (2100, 4096)]:
+        x = torch.ones((h, w), dtype=t_in, device=cuda)
+        flat = torch.full((h * w + 2 * guard,), 7, dtype=torch.int32, device=cuda)
+        out = flat[guard:-guard].view(h, w)
+        ref = (torch.arange(1, h + 1, device=cuda)[:, None] * torch.arange(1, w + 1, device=cuda)[None, :]).to(torch.int32)
+        torch.cuda.synchronize()
+        try:
+            sat_gb300.set_config(cfg)
+            for rev in (False, True):
+                sat_gb300.set_wait_limit_us(1)
+                tiles = ((h + 31) // 32) * ((w + 63) // 64)
+                for tile in (0, tiles - 1, 1):
+                    assert L.satgb_debug_stall_tile(tile) == 0
+                    for _ in range(5):
+                        with torch.cuda.stream(s):
+                            sat_gb300.sat(x, t_out, reverse=rev, out=out.view(t_out))
+                try:
+                    sat_gb300.stream_check(s)
+                except sat_gb300.SatError as e:
+                    assert e.status == _lib.ERR_TIMEOUT
+                assert bool((flat[:guard] == 7).all()) and bool((flat[-guard:] == 7).all())
+                L.satgb_debug_stall_tile(-1)
+                sat_gb300.set_wait_limit_us(2_000_000)
+                with torch.cuda.stream(s):
+                    sat_gb300.sat(x, t_out, reverse=rev, out=out.view(t_out))
+                sat_gb300.stream_check(s)
+                got = out.view(torch.float32).to(torch.int32) if t_out == torch.float32 else out
+                assert torch.equal(got, ref.flip((0, 1)) if rev else ref), (h, w, rev)
+        finally:
+            L.satgb_debug_stall_tile(-1)
+            sat_gb300.set_wait_limit_us(2_000_000)
+            sat_gb300.set_config(-1)
