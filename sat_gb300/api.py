@@ -284,10 +284,15 @@ def box_means(x: torch.Tensor, radii: Sequence[int], out=None, stream=None) -> t
     L = _lib.load()
     st = L.satgb_box_filter_fwd_x(ctypes.byref(d), dx, pitch, plane, _call_stream(stream))
     if st == _lib.ERR_NOT_FOUND:
-        scratch = torch.empty(x.shape, dtype=torch.float32, device=x.device)
-        s3 = scratch if scratch.dim() >= 3 else scratch.unsqueeze(0)
-        d.d_sat, d.sat_pitch, _, _, _, d.sat_plane_stride = _planes_args(s3)
-        st = L.satgb_box_filter_fwd_x(ctypes.byref(d), dx, pitch, plane, _call_stream(stream))
+        # from the pool of the stream that uses it: the block goes back, and to its next owner, in that
+        # stream's order, whatever stream is current
+        handle = _call_stream(stream)
+        scratch = torch.cuda.caching_allocator_alloc(4 * x.numel(), x.device, handle)
+        try:
+            d.d_sat, d.sat_pitch, d.sat_plane_stride = scratch, d.width, d.width * d.height
+            st = L.satgb_box_filter_fwd_x(ctypes.byref(d), dx, pitch, plane, handle)
+        finally:
+            torch.cuda.caching_allocator_delete(scratch)
     check(st)
     return out
 

@@ -369,3 +369,28 @@ def test_box_layer_views_and_offsets(cuda):
         for k, r in enumerate((3, 9)):
             assert float((m[:, k].double() - ref[:, k]).abs().max()) <= window_error(r)
         assert bool(torch.isnan(out[..., w:]).all())
+
+
+def test_box_means_scratch_belongs_to_the_stream(cuda):
+    """The scratch SAT of radii too large for one launch, on a stream that is not the current one: a block that
+    the current stream still writes is not taken for it, and none of it is handed to the current
+    stream while the call's launches are to come."""
+    g = torch.Generator(device="cpu").manual_seed(41)
+    x = torch.randn((6, 500, 600), generator=g).to(cuda)
+    want = api.box_means(x, (80,))
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    for _ in range(3):
+        old = torch.empty_like(x)
+        torch.cuda._sleep(20_000_000)
+        old.fill_(float("nan"))  # after the sleep
+        del old
+        with torch.cuda.stream(side):
+            out = torch.zeros_like(want)
+            torch.cuda._sleep(5_000_000)
+        api.box_means(x, (80,), out=out, stream=side)
+        late = [torch.full_like(x, float("nan")) for _ in range(4)]
+        torch.cuda.synchronize()
+        # (the SAT's sums may differ in their last bits: 2^-24 of |S| < 1e4 over windows of 41 x 41 at least)
+        assert float((out - want).abs().max()) <= 1e-5
+        assert all(bool(torch.isnan(t).all()) for t in late)
