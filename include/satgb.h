@@ -196,10 +196,11 @@ typedef struct {
 satgb_status satgb_box_filter_fwd(const satgb_box_desc* desc, satgb_stream stream);
 /* Box means of every radius straight from the image d_x (n_planes planes of
  * width x height f32, pitch and plane stride in elements), in one launch that
- * writes no SAT.  desc->d_sat (with its pitch and plane stride) is a scratch
- * SAT for radii too large for that kernel's shared memory (above 64, or their
- * planes narrower than their windows); without one (NULL) such a call returns
- * SATGB_ERR_NOT_FOUND.  The means may not overlap the image. */
+ * writes no SAT.  Without a scratch SAT (desc->d_sat NULL) every set of radii up
+ * to 64 is taken so, and larger ones (as clamped to max(width, height) - 1)
+ * return SATGB_ERR_NOT_FOUND.  With one (d_sat with its pitch and plane stride) the call
+ * takes any radii, and goes through the SAT where that is the faster way.
+ * The means may not overlap the image. */
 satgb_status satgb_box_filter_fwd_x(const satgb_box_desc* desc, const void* d_x, int64_t x_pitch,
                                     int64_t x_plane_stride, satgb_stream stream);
 /* The adjoint of satgb_box_filter_fwd: dL/dSAT from the gradients of all the

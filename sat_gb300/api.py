@@ -272,28 +272,31 @@ def box_means_from_sat(sat_t: torch.Tensor, radii: Sequence[int], out=None, stre
     return out
 
 
+# Radii from which the library may go through a SAT (box_fused.cu: two radii of 34 leave an SM two
+# blocks); up to there a scratch SAT would be allocated for nothing.
+_SCRATCH_RADIUS = 34
+
+
 def box_means(x: torch.Tensor, radii: Sequence[int], out=None, stream=None) -> torch.Tensor:
     """Clipped box means of every radius of the image x itself: (..., H, W) ->
-    (..., R, H, W), in one launch; radii too large for that launch go through
-    the SAT of x in a scratch tensor."""
+    (..., R, H, W), in one launch, or for large radii, where that is faster, through
+    the SAT of x in scratch memory."""
     if out is None:
         out = torch.empty(x.shape[:-2] + (len(radii),) + x.shape[-2:], dtype=torch.float32, device=x.device)
     d = _box_desc(x, out, radii)
     dx, pitch, plane = d.d_sat, d.sat_pitch, d.sat_plane_stride
     d.d_sat = None
-    L = _lib.load()
-    st = L.satgb_box_filter_fwd_x(ctypes.byref(d), dx, pitch, plane, _call_stream(stream))
-    if st == _lib.ERR_NOT_FOUND:
+    fwd, handle, scratch = _lib.load().satgb_box_filter_fwd_x, _call_stream(stream), None
+    if min(max(d.radius), max(d.width, d.height) - 1) >= _SCRATCH_RADIUS:
         # from the pool of the stream that uses it: the block goes back, and to its next owner, in that
         # stream's order, whatever stream is current
-        handle = _call_stream(stream)
         scratch = torch.cuda.caching_allocator_alloc(4 * x.numel(), x.device, handle)
-        try:
-            d.d_sat, d.sat_pitch, d.sat_plane_stride = scratch, d.width, d.width * d.height
-            st = L.satgb_box_filter_fwd_x(ctypes.byref(d), dx, pitch, plane, handle)
-        finally:
+        d.d_sat, d.sat_pitch, d.sat_plane_stride = scratch, d.width, d.width * d.height
+    try:
+        check(fwd(ctypes.byref(d), dx, pitch, plane, handle))
+    finally:
+        if scratch is not None:
             torch.cuda.caching_allocator_delete(scratch)
-    check(st)
     return out
 
 

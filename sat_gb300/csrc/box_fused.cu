@@ -436,6 +436,7 @@ int device_sms() {
 }
 
 constexpr int kMaxSmem = 232448; // a block's limit
+constexpr int kMaxRadius = 64;    // (96 output columns a block are left)
 
 // Shared memory of a block: the prefix rows and the rings.
 int64_t means_smem(const BoxArgs& a, int ahead) {
@@ -529,11 +530,12 @@ cudaError_t launch_grad(const BoxArgs& a, const Shape& sh, int smem, cudaStream_
 //             2: radii 3, 31 144 / 152     3: radius 31 100 / 121
 namespace satgb {
 
-satgb_status box_means_fused(const BoxArgs& a, cudaStream_t s, bool* done) {
+satgb_status box_means_fused(const BoxArgs& a, cudaStream_t s, bool only_way, bool* done) {
   Shape sh;
   int64_t smem = means_smem(a, sh.ahead = 1);
+  static_assert((kPMeans * SATGB_MAX_RADII + 2 * kMaxRadius + 1 + 2 * kDMeans) * kW * 4 <= kMaxSmem, "a block fits");
   const int blocks = resident(smem);
-  *done = a.rmax <= 64 && (blocks >= 3 || (blocks == 2 && a.nr >= 3));
+  *done = a.rmax <= kMaxRadius && (only_way || blocks >= 3 || (blocks == 2 && a.nr >= 3));
   if (!*done) return SATGB_OK;
   if (resident(means_smem(a, 2)) == blocks) smem = means_smem(a, sh.ahead = 2);
   sh.tx = columns(a);
@@ -550,7 +552,7 @@ satgb_status box_grad_fused(const BoxArgs& a, cudaStream_t s, bool* done) {
   Shape sh;
   int64_t smem = grad_smem(a, sh.ahead = 1);
   const int blocks = resident(smem);
-  *done = a.rmax <= 64 && smem <= kMaxSmem && (blocks >= 3 || (blocks == 2 && a.nr >= 2) || a.nr == 4);
+  *done = a.rmax <= kMaxRadius && smem <= kMaxSmem && (blocks >= 3 || (blocks == 2 && a.nr >= 2) || a.nr == 4);
   if (!*done) return SATGB_OK;
   if (resident(grad_smem(a, 2)) == blocks && grad_smem(a, 2) <= kMaxSmem) smem = grad_smem(a, sh.ahead = 2);
   sh.tx = columns(a);

@@ -1041,10 +1041,10 @@ satgb_status satgb_box_filter_fwd_x(const satgb_box_desc* desc, const void* d_x,
       return fail(SATGB_ERR_INVALID_ARG, "box means: the means overlap the image");
   }
   bool done = false;
-  st = satgb::box_means_fused(a, (cudaStream_t)stream, &done);
+  st = satgb::box_means_fused(a, (cudaStream_t)stream, !desc->d_sat, &done);
   if (st != SATGB_OK || done) return st;
   if (!desc->d_sat)
-    return fail(SATGB_ERR_NOT_FOUND, "box means: these radii need a scratch SAT (descriptor's d_sat)");
+    return fail(SATGB_ERR_NOT_FOUND, "box means: radii above 64 need a scratch SAT (descriptor's d_sat)");
   const long long splane = planes > 1 ? desc->sat_plane_stride : 0;
   if (desc->sat_pitch < w || (planes > 1 && splane < (h - 1) * desc->sat_pitch + w))
     return fail(SATGB_ERR_INVALID_ARG, "box means: scratch SAT pitch or plane stride too small");

@@ -394,3 +394,32 @@ def test_box_means_scratch_belongs_to_the_stream(cuda):
         # (the SAT's sums may differ in their last bits: 2^-24 of |S| < 1e4 over windows of 41 x 41 at least)
         assert float((out - want).abs().max()) <= 1e-5
         assert all(bool(torch.isnan(t).all()) for t in late)
+
+
+@pytest.mark.parametrize("radii", [(34,), (35,), (40,), (64,), (33, 34), (3, 7, 52), (50, 51, 52, 64), (64, 64, 64, 64)])
+def test_box_means_without_a_scratch_sat(cuda, radii):
+    """The C call takes every set of radii up to 64 without a scratch SAT; above, where the image is
+    large enough for them, it says that it needs one."""
+    import ctypes
+    L = sat_gb300._lib.load()
+    g = torch.Generator(device="cpu").manual_seed(43)
+    x = torch.randn((2, 150, 170), generator=g).to(cuda)
+    out = torch.empty((2, len(radii), 150, 170), device=cuda)
+
+    def call(radii, width):
+        d = api._box_desc(x[..., :width], out[..., :width], radii)
+        dx, pitch, plane = d.d_sat, d.sat_pitch, d.sat_plane_stride
+        d.d_sat = None
+        return L.satgb_box_filter_fwd_x(ctypes.byref(d), dx, pitch, plane, torch.cuda.current_stream().cuda_stream)
+
+    assert call(radii, 170) == sat_gb300._lib.OK
+    ref = box_means64(x, radii)
+    for k, r in enumerate(radii):
+        assert float((out[:, k].double() - ref[:, k]).abs().max()) <= window_error(r)
+    assert call(radii[:-1] + (65,), 170) == sat_gb300._lib.ERR_NOT_FOUND
+    x = x[:, :65].contiguous()  # radius 65 and above are the whole image here: 64
+    out = torch.empty((2, len(radii), 65, 170), device=cuda)
+    assert call(radii[:-1] + (1000,), 60) == sat_gb300._lib.OK
+    ref = box_means64(x[..., :60], radii[:-1] + (1000,))
+    for k, r in enumerate(radii[:-1] + (64,)):
+        assert float((out[:, k, :, :60].double() - ref[:, k]).abs().max()) <= window_error(min(r, 29))
