@@ -12,7 +12,10 @@
 //   window    = p_k(y, x + r_k) - p_k(y, x - r_k - 1)               through shared memory
 //
 // Every sum starts inside the strip, so its rounding errors are those of sums of
-// a few hundred elements instead of those of a whole plane's SAT.
+// a few hundred elements instead of those of a whole plane's SAT.  An infinity or
+// NaN stays in the sums that pass it, to the end of the strip and of the block, so
+// each kernel runs the way its SAT does, the gradient from the last row and column
+// back: what it spoils the way through the SAT spoils too.
 //
 // A block owns a strip of sy rows of kW = 256 prefix columns, of which tx (host:
 // columns) are output columns and the rest the windows' reach to both sides, and has one
@@ -76,12 +79,17 @@ __device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
   return r;
 }
 
-// v += the value D lanes below, where there is one
-template <int D>
-__device__ __forceinline__ void add_from_below(float& v) {
-  asm("{\n\t.reg .pred p;\n\t.reg .f32 t;\n\tshfl.sync.up.b32 t|p, %0, %1, 0, 0xffffffff;\n\t@p add.rn.f32 %0, %0, t;\n\t}"
-      : "+f"(v)
-      : "n"(D));
+// v += the value D lanes below (REV: above), where there is one
+template <bool REV, int D>
+__device__ __forceinline__ void add_across(float& v) {
+  if constexpr (REV)
+    asm("{\n\t.reg .pred p;\n\t.reg .f32 t;\n\tshfl.sync.down.b32 t|p, %0, %1, 31, 0xffffffff;\n\t@p add.rn.f32 %0, %0, t;\n\t}"
+        : "+f"(v)
+        : "n"(D));
+  else
+    asm("{\n\t.reg .pred p;\n\t.reg .f32 t;\n\tshfl.sync.up.b32 t|p, %0, %1, 0, 0xffffffff;\n\t@p add.rn.f32 %0, %0, t;\n\t}"
+        : "+f"(v)
+        : "n"(D));
 }
 
 __device__ __forceinline__ float clipped_inv(int i, int r, int n, float inv_full) {
@@ -134,8 +142,9 @@ __device__ __forceinline__ void ring_read(F2 (&v)[4], const float* row, int d) {
 }
 
 // The prefix sums of D rows whose elements the warp holds, 8 adjacent ones a lane, into shared memory rows
-// `pitch` apart.  The rows go side by side: a row alone is one long chain of shuffles.
-template <int D>
+// `pitch` apart; REV: for each column the sum of those after it.  The rows go side by side: a row alone is one long
+// chain of shuffles.
+template <int D, bool REV = false>
 __device__ __forceinline__ void prefix_rows(const F2 (&u)[D][4], float* dst, int pitch, int d, int lane) {
   float a[D], b[D], incl[D]; // the chunks' sums
 #pragma unroll
@@ -148,28 +157,41 @@ __device__ __forceinline__ void prefix_rows(const F2 (&u)[D][4], float* dst, int
     incl[i] = a[i] + b[i];
   }
 #pragma unroll
-  for (int i = 0; i < D; ++i) add_from_below<1>(incl[i]);
+  for (int i = 0; i < D; ++i) add_across<REV, 1>(incl[i]);
 #pragma unroll
-  for (int i = 0; i < D; ++i) add_from_below<2>(incl[i]);
+  for (int i = 0; i < D; ++i) add_across<REV, 2>(incl[i]);
 #pragma unroll
-  for (int i = 0; i < D; ++i) add_from_below<4>(incl[i]);
+  for (int i = 0; i < D; ++i) add_across<REV, 4>(incl[i]);
 #pragma unroll
-  for (int i = 0; i < D; ++i) add_from_below<8>(incl[i]);
+  for (int i = 0; i < D; ++i) add_across<REV, 8>(incl[i]);
 #pragma unroll
-  for (int i = 0; i < D; ++i) add_from_below<16>(incl[i]);
+  for (int i = 0; i < D; ++i) add_across<REV, 16>(incl[i]);
 #pragma unroll
   for (int i = 0; i < D; ++i) {
-    float ex = __shfl_up_sync(0xffffffffu, incl[i], 1);
-    if (lane == 0) ex = 0.f;
+    float ex = REV ? __shfl_down_sync(0xffffffffu, incl[i], 1) : __shfl_up_sync(0xffffffffu, incl[i], 1);
+    if (lane == (REV ? 31 : 0)) ex = 0.f;
     float v[8];
 #pragma unroll
     for (int q = 0; q < 4; ++q) unpack(u[i][q], v[2 * q], v[2 * q + 1]);
-    v[0] += d < 0 ? ex + b[i] : ex;
-    v[4] += d < 0 ? ex : ex + a[i];
+    if constexpr (REV) {
+      // sums of the columns after: each chunk's last column has what comes after the chunk
+      float ra = d < 0 ? ex : ex + b[i], rb = d < 0 ? ex + a[i] : ex;
 #pragma unroll
-    for (int q = 1; q < 4; ++q) {
-      v[q] += v[q - 1];
-      v[q + 4] += v[q + 3];
+      for (int q = 3; q >= 0; --q) {
+        const float na = v[q] + ra, nb = v[q + 4] + rb;
+        v[q] = ra;
+        v[q + 4] = rb;
+        ra = na;
+        rb = nb;
+      }
+    } else {
+      v[0] += d < 0 ? ex + b[i] : ex;
+      v[4] += d < 0 ? ex : ex + a[i];
+#pragma unroll
+      for (int q = 1; q < 4; ++q) {
+        v[q] += v[q - 1];
+        v[q + 4] += v[q + 3];
+      }
     }
     *reinterpret_cast<float4*>(dst + i * pitch) = make_float4(v[0], v[1], v[2], v[3]);
     *reinterpret_cast<float4*>(dst + i * pitch + d) = make_float4(v[4], v[5], v[6], v[7]);
@@ -326,11 +348,11 @@ __global__ void __launch_bounds__(NR * 32) box_grad_kernel(const __grid_constant
     if (i < k) ring += (2 * a.r[i] + 1 + (1 + sh.ahead) * D) * kW;
   const int wrap = (2 * r + 1 + (1 + sh.ahead) * D) * kW;
   const float* src = a.box[k] + (int64_t)blockIdx.z * a.box_plane;
-  int jn = y0 - r - 1, jslot = 0;
+  int jn = y1 + r, jslot = 0;
   auto copy = [&](int n) {
-    if (jn < y1 + r) {
-      for (int i = 0; i < n; ++i, ++jn) {
-        copy_row<VEC, 32>(ring + jslot, src + (int64_t)jn * a.box_pitch, src, xs, W, jn >= 0 && jn < min(H, y1 + r), lane);
+    if (jn >= y0 - r) {
+      for (int i = 0; i < n; ++i, --jn) {
+        copy_row<VEC, 32>(ring + jslot, src + (int64_t)jn * a.box_pitch, src, xs, W, jn >= max(0, y0 - r) && jn < H, lane);
         jslot += kW;
         if (jslot == wrap) jslot = 0;
       }
@@ -365,9 +387,9 @@ __global__ void __launch_bounds__(NR * 32) box_grad_kernel(const __grid_constant
     const int i = (t0 + t) / ng, c = (t0 + t) - i * ng;
     pi[t] = t < nt && c * 32 + lane < n ? i : H;
     ps[t] = t < nt ? i * (NR * kW) + c * 32 : 0;
-    po[t] = c * 32 + i * a.sat_pitch;
+    po[t] = c * 32 - i * a.sat_pitch;
   }
-  float* out = a.sat + (int64_t)blockIdx.z * a.sat_plane + (int64_t)y0 * a.sat_pitch + X0 + lane;
+  float* out = a.sat + (int64_t)blockIdx.z * a.sat_plane + (int64_t)(y1 - 1) * a.sat_pitch + X0 + lane;
 
   F2 V[4];
 #pragma unroll
@@ -375,30 +397,30 @@ __global__ void __launch_bounds__(NR * 32) box_grad_kernel(const __grid_constant
   int sout = 0, sin = (2 * r + 1) * kW;
   copies_wait_ahead(sh.ahead);
   __syncthreads();
-  for (int i = 0; i <= 2 * r; ++i) { // the window of row y0 - 1
+  for (int i = 0; i <= 2 * r; ++i) { // the window of row y1
     F2 e[4];
     ring_read(e, mine + i * kW, d);
-    const float f = clipped_inv(min(max(y0 - r - 1 + i, 0), H - 1), r, H, inv);
+    const float f = clipped_inv(min(max(y1 + r - i, 0), H - 1), r, H, inv);
 #pragma unroll
     for (int q = 0; q < 4; ++q) V[q] = fma2(f2(f, f), e[q], V[q]);
   }
 #pragma unroll 1
-  for (int yb = y0; yb < y1; yb += D) {
+  for (int yb = y1 - 1; yb >= y0; yb -= D) {
     copies_wait_ahead(sh.ahead - 1);
     __syncthreads(); // the last batch's prefix rows have been read; this batch's rows have arrived
     copy(D);
-    const bool yinner = yb - 2 * r - 1 >= 0 && yb + D - 1 + 2 * r <= H - 1;
+    const bool yinner = yb - (D - 1) - 2 * r >= 0 && yb + 2 * r + 1 <= H - 1;
     F2 u[D][4];
 #pragma unroll
     for (int i = 0; i < D; ++i) {
-      const int y = yb + i;
+      const int y = yb - i;
       F2 e[4], l[4];
       ring_read(e, mine + sin, d);
       ring_read(l, mine + sout, d);
       float fe = inv, fl = inv;
       if (!yinner) {
-        fe = clipped_inv(min(max(y + r, 0), H - 1), r, H, inv);
-        fl = clipped_inv(min(max(y - r - 1, 0), H - 1), r, H, inv);
+        fe = clipped_inv(min(max(y - r, 0), H - 1), r, H, inv);
+        fl = clipped_inv(min(max(y + r + 1, 0), H - 1), r, H, inv);
       }
 #pragma unroll
       for (int q = 0; q < 4; ++q) V[q] = fma2(f2(-fl, -fl), l[q], fma2(f2(fe, fe), e[q], V[q]));
@@ -409,17 +431,17 @@ __global__ void __launch_bounds__(NR * 32) box_grad_kernel(const __grid_constant
 #pragma unroll
       for (int q = 0; q < 4; ++q) u[i][q] = mul2(V[q], ix[q]);
     }
-    prefix_rows<D>(u, wr, NR * kW, d, lane);
+    prefix_rows<D, true>(u, wr, NR * kW, d, lane);
     __syncthreads();
 #pragma unroll
     for (int t = 0; t < T; ++t) {
       if (t >= nt) break;
-      float s = rd[0][ps[t]] - ld[0][ps[t]];
+      float s = ld[0][ps[t]] - rd[0][ps[t]];
 #pragma unroll
-      for (int q = 1; q < NR; ++q) s += rd[q][ps[t]] - ld[q][ps[t]];
-      if (yb + pi[t] < y1) __stcs(out + po[t], s);
+      for (int q = 1; q < NR; ++q) s += ld[q][ps[t]] - rd[q][ps[t]];
+      if (yb - pi[t] >= y0) __stcs(out + po[t], s);
     }
-    out += D * a.sat_pitch;
+    out -= D * a.sat_pitch;
   }
 }
 

@@ -423,3 +423,42 @@ def test_box_means_without_a_scratch_sat(cuda, radii):
     ref = box_means64(x[..., :60], radii[:-1] + (1000,))
     for k, r in enumerate(radii[:-1] + (64,)):
         assert float((out[:, k, :, :60].double() - ref[:, k]).abs().max()) <= window_error(min(r, 29))
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan")])
+@pytest.mark.parametrize("shape,radii", [((1, 300, 700), (3, 7, 15)), ((2, 150, 333), (5,)), ((1, 70, 64), (1, 9, 20, 31))])
+def test_box_layer_infinities_spoil_no_more_than_the_sat_path(cuda, shape, radii, value):
+    """An infinity or NaN in x spoils means whose window's last row and column are not before it only (those
+    the SAT's four corners take it into), one in the means' gradient the pixels up to its window's last
+    row and column only (the reverse SAT's); every other element is what it is without it, and every
+    mean whose window holds it is not finite."""
+    g = torch.Generator(device="cpu").manual_seed(47)
+    x = torch.randn(shape, generator=g).to(cuda)
+    w = torch.randn(shape[:-2] + (len(radii),) + shape[-2:], generator=g).to(cuda)
+    H, W = shape[-2:]
+    ys = torch.arange(H, device=cuda)[:, None]
+    xs = torch.arange(W, device=cuda)[None, :]
+    m64 = box_means64(x, radii)
+    x64 = x.double().requires_grad_(True)
+    (dx64,) = torch.autograd.grad(box_means64(x64, radii), x64, w.double())
+    for r0, c0 in [(H // 2, W // 3), (0, 0), (H - 1, W - 1), (H // 3, W - 2), (H - 2, 5)]:
+        x2 = x.clone()
+        x2[0, r0, c0] = value
+        m = api.box_means(x2, radii)
+        for k, r in enumerate(radii):
+            sound = ((ys + r).clamp(max=H - 1) < r0) | ((xs + r).clamp(max=W - 1) < c0)
+            err = (m[0, k].double() - m64[0, k]).abs()
+            assert bool((err[sound] <= window_error(r)).all()), (r0, c0, r)
+            holds = ((ys - r0).abs() <= r) & ((xs - c0).abs() <= r)
+            assert not bool(m[0, k][holds].isfinite().any()), (r0, c0, r)
+        for k, r in enumerate(radii):
+            w2 = w.clone()
+            w2[0, k, r0, c0] = value
+            dx = api.box_means_grad_x(w2, radii)
+            sound = (ys > r0 + r) | (xs > c0 + r)
+            err = (dx[0].double() - dx64[0]).abs()
+            assert bool((err[sound] <= sum(window_error(q) for q in radii)).all()), (r0, c0, r)
+            holds = ((ys - r0).abs() <= r) & ((xs - c0).abs() <= r)
+            assert not bool(dx[0][holds].isfinite().any()), (r0, c0, r)
+        for i in range(1, shape[0]):
+            assert bool(m[i].isfinite().all()) and bool(dx[i].isfinite().all())
