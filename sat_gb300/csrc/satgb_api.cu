@@ -464,7 +464,7 @@ satgb_status check_batch_disjoint(const std::vector<ImgCheck>& imgs, size_t in_s
 // ----------------------------------------------------------------------------
 using TuneKey = std::tuple<int, int, int, int, int, int, int>;
 std::map<TuneKey, int> g_tune;
-// batch plans: (in, out, mode, dir, size class, log2 pixels, log2 images, all rows TMA-able, SMs) -> cfg
+// batch plans: (in, out, mode, dir, size class, log2 pixels, log2 images, rows (batch_key), SMs) -> cfg
 using BatchKey = std::tuple<int, int, int, int, int, int, int, int, int>;
 std::map<BatchKey, int> g_batch_tune;
 bool g_tune_loaded = false;
@@ -771,7 +771,8 @@ constexpr long long kLargeTiles = 64; // an image of at least 64 tiles of 128 x 
 
 struct BatchSeg {
   const Variant* v = nullptr;
-  std::vector<ImgCheck> imgs;
+  std::vector<ImgCheck> imgs; // as the caller gave them
+  std::vector<ImgCheck> src;  // as the kernel reads them (staged inputs: their copies)
   long long n_images = 0, n_tiles = 0;
   double pixels = 0;
   ImageDesc img0;
@@ -784,6 +785,7 @@ struct satgb_batch_plan_s {
   int in_t = 0, out_t = 0, mode = 0, dir = 0;
   int dev = 0;
   bool all_tma = true; // every image's rows can go through TMA (16-byte aligned bases and pitches)
+  bool off16 = false;  // some inputs are off 16-byte boundaries: TMA reads copies of them, or groups of rows
   // Inputs whose rows TMA cannot address are copied at each execution into
   // padded rows of `stage` (batch_repack.cu); `jobs` (device) lists them.
   void* stage = nullptr;
@@ -1101,10 +1103,12 @@ satgb_status satgb_box_filter_bwd_x(const satgb_box_desc* desc, void* d_dx, int6
 
 namespace {
 
+// The rows' part of the key: 1 as all_tma, and 2 for inputs off 16-byte boundaries, which some configurations
+// read as they are and others as copies made at each execution.
 BatchKey batch_key(const satgb_batch_plan_s* p, int cls, int sms) {
   const BatchSeg& g = p->seg[cls];
   return BatchKey(p->in_t, p->out_t, p->mode, p->dir, cls, log2_bucket((long long)std::max(1.0, g.pixels)),
-                  log2_bucket(std::max(1LL, g.n_images)), p->all_tma ? 1 : 0, sms);
+                  log2_bucket(std::max(1LL, g.n_images)), (p->all_tma ? 1 : 0) + (p->off16 ? 2 : 0), sms);
 }
 
 // Untuned choice for a class: 1-byte images of every size the packed tiles of
@@ -1181,7 +1185,7 @@ satgb_status seg_build(satgb_batch_plan_s* p, BatchSeg& g, const Variant* v, cud
   if (!v) return fail(SATGB_ERR_UNSUPPORTED_TYPES, "no kernel for this batch");
   std::vector<ImageDesc> table;
   long long base = 0;
-  for (auto& c : g.imgs) {
+  for (auto& c : g.src) {
     ImageDesc d;
     fill_image_desc(d, v, p->in_t, p->out_t, c.in, c.out, c.in_pitch, c.out_pitch, c.width, c.height, base, 1, 0, 0);
     base += (long long)d.ntx * d.nty;
@@ -1217,7 +1221,7 @@ satgb_status plan_merge(satgb_batch_plan_s* p, cudaStream_t s) {
   for (auto& g : p->seg)
     if (!g.n_tiles || g.v != p->seg[0].v) return SATGB_OK;
   for (auto& g : p->seg) {
-    p->all.imgs.insert(p->all.imgs.end(), g.imgs.begin(), g.imgs.end());
+    p->all.src.insert(p->all.src.end(), g.src.begin(), g.src.end());
     p->all.n_images += g.n_images;
   }
   return seg_build(p, p->all, p->seg[0].v, s);
@@ -1262,12 +1266,16 @@ satgb_status plan_launch_locked(satgb_batch_plan_s* p, cudaStream_t s) {
   return SATGB_OK;
 }
 
-// Captures the classes' launches, one after the other, in the plan's graph.
-satgb_status plan_capture(satgb_batch_plan_s* p) {
+void plan_uncapture(satgb_batch_plan_s* p) {
   if (p->exec) cudaGraphExecDestroy(p->exec);
   if (p->graph) cudaGraphDestroy(p->graph);
   p->exec = nullptr;
   p->graph = nullptr;
+}
+
+// Captures the classes' launches, one after the other, in the plan's graph.
+satgb_status plan_capture(satgb_batch_plan_s* p) {
+  plan_uncapture(p);
   cudaStream_t cs;
   cudaError_t e = cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking);
   if (e != cudaSuccess) return cuda_fail(e, "cudaStreamCreate");
@@ -1291,8 +1299,7 @@ satgb_status plan_capture(satgb_batch_plan_s* p) {
 }
 
 void plan_free(satgb_batch_plan_s* p) {
-  if (p->exec) cudaGraphExecDestroy(p->exec);
-  if (p->graph) cudaGraphDestroy(p->graph);
+  plan_uncapture(p);
   ws_free(p->ws.base);
   ws_free(p->stage);
   if (p->jobs) cudaFree(p->jobs);
@@ -1305,8 +1312,8 @@ void plan_free(satgb_batch_plan_s* p) {
 // least 16 bytes a row), and whose class's kernel (`vs`) does not read packed rows
 // through TMA as they are, get a copy in padded rows: the plan's staging buffer,
 // one region per image (256-byte aligned, rows of the width rounded up to 16
-// bytes), and the tile kernels read the copies.  Rewrites the images' input
-// pointers and pitches.
+// bytes), and the tile kernels read the copies.  Fills the classes' `src`, in place of
+// an earlier choice of kernels; a class without a kernel (nullptr) is not staged.
 satgb_status plan_stage_inputs(satgb_batch_plan_s* p, const Variant* const (&vs)[kBatchClasses], size_t in_sz,
                                cudaStream_t s) {
   std::vector<satgb::RepackJob> jobs;
@@ -1314,14 +1321,27 @@ satgb_status plan_stage_inputs(satgb_batch_plan_s* p, const Variant* const (&vs)
   std::vector<ImgCheck*> which;
   size_t total = 0;
   long long rows = 0;
+  if (p->stage || p->jobs) {
+    const cudaError_t e = cudaStreamSynchronize(s); // earlier launches may still read them
+    if (e != cudaSuccess) return cuda_fail(e, "cudaStreamSynchronize");
+    ws_free(p->stage);
+    if (p->jobs) cudaFree(p->jobs);
+    p->stage = nullptr;
+    p->jobs = nullptr;
+    p->n_jobs = 0;
+    p->stage_rows = 0;
+  }
   std::vector<std::pair<ImgCheck*, const Variant*>> imgs;
-  for (int cls = 0; cls < kBatchClasses; ++cls)
-    for (ImgCheck& c : p->seg[cls].imgs) imgs.emplace_back(&c, vs[cls]);
+  for (int cls = 0; cls < kBatchClasses; ++cls) {
+    p->seg[cls].src = p->seg[cls].imgs;
+    if (vs[cls])
+      for (ImgCheck& c : p->seg[cls].src) imgs.emplace_back(&c, vs[cls]);
+  }
   for (auto& [img, v] : imgs) {
     ImgCheck& c = *img;
     const size_t row_bytes = (size_t)c.width * in_sz;
     if (row_bytes < 16 || tma_ok(c.in, c.width, c.height, c.in_pitch, 1, 0, in_sz)) continue;
-    if (v && skew_rows(v, c.in, c.in_pitch, c.width, c.height, 1, in_sz)) continue;
+    if (skew_rows(v, c.in, c.in_pitch, c.width, c.height, 1, in_sz)) continue;
     const size_t pitch = (row_bytes + 15) & ~(size_t)15;
     satgb::RepackJob j;
     j.src = static_cast<const unsigned char*>(c.in);
@@ -1356,6 +1376,39 @@ satgb_status plan_stage_inputs(satgb_batch_plan_s* p, const Variant* const (&vs)
   p->n_jobs = (int)jobs.size();
   p->stage_rows = rows;
   return SATGB_OK;
+}
+
+// Lays the plan out for its classes' kernels (nullptr: the class stays out): staged inputs, tables,
+// workspace.  Called with g_mu held.
+satgb_status plan_layout(satgb_batch_plan_s* p, const Variant* const (&vs)[kBatchClasses], cudaStream_t s) {
+  satgb_status st = plan_stage_inputs(p, vs, dtype_size(p->in_t), s);
+  for (int cls = 0; cls < kBatchClasses && st == SATGB_OK; ++cls) {
+    BatchSeg& g = p->seg[cls];
+    if (vs[cls]) {
+      st = seg_build(p, g, vs[cls], s);
+    } else {
+      seg_free(g);
+      g.n_tiles = 0;
+    }
+  }
+  if (st == SATGB_OK) st = plan_merge(p, s);
+  if (st == SATGB_OK) st = plan_ws(p, s);
+  return st;
+}
+
+// Time of one execution of the plan as it is laid out, copies included.
+satgb_status plan_time(satgb_batch_plan_s* p, cudaStream_t s, cudaEvent_t e0, cudaEvent_t e1, float* ms) {
+  const int warm = 2, reps = 5;
+  satgb_status st = SATGB_OK;
+  for (int i = 0; i < warm + reps && st == SATGB_OK; ++i) {
+    if (i == warm) cudaEventRecord(e0, s);
+    st = plan_launch_locked(p, s);
+  }
+  cudaEventRecord(e1, s);
+  const cudaError_t e = cudaEventSynchronize(e1);
+  if (st == SATGB_OK && e != cudaSuccess) st = cuda_fail(e, "cudaEventSynchronize");
+  if (st == SATGB_OK) cudaEventElapsedTime(ms, e0, e1);
+  return st;
 }
 
 }  // namespace
@@ -1404,9 +1457,10 @@ satgb_status satgb_batch_plan_create(satgb_batch_plan** plan, satgb_dtype in_t, 
     g.n_images += 1;
     g.pixels += (double)c.width * (double)c.height;
     // (rows of 16 bytes and more that are not are staged, or the kernel reads them through TMA as they are)
+    const bool on16 = ((uintptr_t)c.in % 16) == 0 && ((size_t)c.in_pitch * in_sz) % 16 == 0;
     p->all_tma = p->all_tma && ((uintptr_t)c.out % 16) == 0 && ((size_t)c.out_pitch * out_sz) % 16 == 0 &&
-                 ((((uintptr_t)c.in % 16) == 0 && ((size_t)c.in_pitch * in_sz) % 16 == 0) ||
-                  (size_t)c.width * in_sz >= 16);
+                 (on16 || (size_t)c.width * in_sz >= 16);
+    p->off16 = p->off16 || !on16;
   }
   tune_load_locked();
   const int sms = sms_of(dev);
@@ -1421,11 +1475,7 @@ satgb_status satgb_batch_plan_create(satgb_batch_plan** plan, satgb_dtype in_t, 
     }
     vs[cls] = seg_variant(p, cls, cfgs[cls]);
   }
-  st = plan_stage_inputs(p, vs, in_sz, s);
-  for (int cls = 0; cls < kBatchClasses && st == SATGB_OK; ++cls)
-    if (p->seg[cls].n_images) st = seg_build(p, p->seg[cls], vs[cls], s);
-  if (st == SATGB_OK) st = plan_merge(p, s);
-  if (st == SATGB_OK) st = plan_ws(p, s);
+  st = plan_layout(p, vs, s);
   if (st == SATGB_OK && p->n_tiles > 0) st = plan_capture(p);
   if (st != SATGB_OK) {
     plan_free(p);
@@ -1444,58 +1494,72 @@ satgb_status satgb_batch_plan_autotune(satgb_batch_plan* p, satgb_stream stream,
   cudaEvent_t e0, e1;
   if (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess)
     return cuda_fail(cudaGetLastError(), "cudaEventCreate");
-  satgb_status st = plan_repack(p, s); // the staged inputs the timed launches read
-  for (int cls = 0; cls < kBatchClasses && st == SATGB_OK; ++cls) {
-    BatchSeg& g = p->seg[cls];
+  // Every candidate is laid out and timed as a plan that takes it would run: with the copies it needs and
+  // no others, and two classes with one kernel as one launch.
+  const Variant* was[kBatchClasses] = {};
+  const Variant* best[kBatchClasses] = {};
+  satgb_status st = SATGB_OK;
+  float ms = 0.f;
+  for (int cls = 0; cls < kBatchClasses; ++cls) {
     if (configs) configs[cls] = -1;
-    if (!g.n_images) continue;
-    int best = -1;
+    if (p->seg[cls].n_images) was[cls] = p->seg[cls].v;
+  }
+  for (int cls = 0; cls < kBatchClasses && st == SATGB_OK; ++cls) {
+    if (!was[cls]) continue;
     float best_ms = 1e30f;
     for (int cfg = 0; cfg < kNumConfigs && st == SATGB_OK; ++cfg) {
-      const Variant* v = find_variant(p->in_t, p->out_t, p->mode, p->dir, cfg);
-      if (!v || v->cfg != cfg) continue;
-      st = seg_build(p, g, v, s);
-      if (st == SATGB_OK) st = plan_ws(p, s);
-      if (st != SATGB_OK) break;
-      for (int i = 0; i < 2 && st == SATGB_OK; ++i)
-        st = launch_locked(g.v, g.table, g.img0, g.n_images, g.n_tiles, p->ws, p->dev, s, g.order, g.skewed);
-      const int reps = 5;
-      cudaEventRecord(e0, s);
-      for (int i = 0; i < reps && st == SATGB_OK; ++i)
-        st = launch_locked(g.v, g.table, g.img0, g.n_images, g.n_tiles, p->ws, p->dev, s, g.order, g.skewed);
-      cudaEventRecord(e1, s);
-      cudaError_t e = cudaEventSynchronize(e1);
-      if (e != cudaSuccess) st = cuda_fail(e, "cudaEventSynchronize");
-      float ms = 0.f;
-      cudaEventElapsedTime(&ms, e0, e1);
+      const Variant* only[kBatchClasses] = {};
+      only[cls] = find_variant(p->in_t, p->out_t, p->mode, p->dir, cfg);
+      if (!only[cls]) continue;
+      st = plan_layout(p, only, s);
+      if (st == SATGB_OK) st = plan_time(p, s, e0, e1, &ms);
       if (st == SATGB_OK && ms < best_ms) {
         best_ms = ms;
-        best = cfg;
+        best[cls] = only[cls];
       }
     }
-    if (st != SATGB_OK) break;
-    st = seg_build(p, g, seg_variant(p, cls, best), s);
-    g_batch_tune[batch_key(p, cls, sms)] = best;
-    if (configs) configs[cls] = best;
+  }
+  if (st == SATGB_OK && best[0] && best[1] && best[0] != best[1]) {
+    const Variant* pairs[3][kBatchClasses] = {{best[0], best[1]}, {best[0], best[0]}, {best[1], best[1]}};
+    float best_ms = 1e30f;
+    for (auto& pair : pairs) {
+      if (st == SATGB_OK) st = plan_layout(p, pair, s);
+      if (st == SATGB_OK) st = plan_time(p, s, e0, e1, &ms);
+      if (st == SATGB_OK && ms < best_ms) {
+        best_ms = ms;
+        std::copy(pair, pair + kBatchClasses, best);
+      }
+    }
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  if (st == SATGB_OK) st = plan_merge(p, s);
-  if (st == SATGB_OK) st = plan_ws(p, s);
+  if (st == SATGB_OK) st = plan_layout(p, best, s);
   if (st == SATGB_OK) {
     WsHeader h;
     cudaError_t e = cudaMemcpy(&h, p->ws.base, sizeof h, cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) st = cuda_fail(e, "cudaMemcpy");
     else if (h.sticky) st = fail(SATGB_ERR_TIMEOUT, "a look-back wait timed out while tuning (tile %u)", h.sticky_tile);
   }
-  if (st == SATGB_OK) tune_save_locked();
-  if (st == SATGB_OK && p->n_tiles > 0) st = plan_capture(p);
+  if (st == SATGB_OK) {
+    for (int cls = 0; cls < kBatchClasses; ++cls) {
+      if (!best[cls]) continue;
+      g_batch_tune[batch_key(p, cls, sms)] = best[cls]->cfg;
+      if (configs) configs[cls] = best[cls]->cfg;
+    }
+    tune_save_locked();
+    return p->n_tiles > 0 ? plan_capture(p) : SATGB_OK;
+  }
+  // the plan stays what it was, unless that fails too
+  const std::string why = g_last_error;
+  if (plan_layout(p, was, s) != SATGB_OK || p->n_tiles == 0 || plan_capture(p) != SATGB_OK) plan_uncapture(p);
+  g_last_error = why;
   return st;
 }
 
 satgb_status satgb_batch_plan_exec(satgb_batch_plan* p, satgb_stream stream) {
   if (!p) return fail(SATGB_ERR_INVALID_ARG, "null plan");
-  if (p->n_tiles == 0) return SATGB_OK;
+  if (p->seg[0].n_images + p->seg[1].n_images == 0) return SATGB_OK;
+  if (!p->exec) return fail(SATGB_ERR_ALLOC, "the plan has no launches left (an autotune failed)");
   cudaError_t e = cudaGraphLaunch(p->exec, (cudaStream_t)stream);
   if (e != cudaSuccess) return cuda_fail(e, "cudaGraphLaunch");
   g_launches.fetch_add((long long)plan_launches(p).size());
@@ -1504,7 +1568,8 @@ satgb_status satgb_batch_plan_exec(satgb_batch_plan* p, satgb_stream stream) {
 
 satgb_status satgb_batch_plan_launch(satgb_batch_plan* p, satgb_stream stream) {
   if (!p) return fail(SATGB_ERR_INVALID_ARG, "null plan");
-  if (p->n_tiles == 0) return SATGB_OK;
+  if (p->seg[0].n_images + p->seg[1].n_images == 0) return SATGB_OK;
+  if (!p->exec) return fail(SATGB_ERR_ALLOC, "the plan has no launches left (an autotune failed)");
   std::lock_guard<std::mutex> lk(g_mu);
   return plan_launch_locked(p, (cudaStream_t)stream);
 }

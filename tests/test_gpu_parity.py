@@ -961,3 +961,73 @@ def test_waits_that_end_early_stay_inside_the_image(cuda, cfg, t_in, t_out):
             L.satgb_debug_stall_tile(-1)
             sat_gb300.set_wait_limit_us(2_000_000)
             sat_gb300.set_config(-1)
+
+
+@pytest.mark.parametrize("first", [2, 5])
+@pytest.mark.parametrize("t_in,t_out", [(torch.uint8, torch.uint32), (torch.float32, torch.float32)])
+def test_autotuned_plan_is_the_plan_its_entry_makes(cuda, tmp_path, monkeypatch, first, t_in, t_out):
+    """A plan of packed rows off 16-byte boundaries holds copies of them or not as the configuration it was
+    tuned to needs them, whichever it was made with: the same as a new plan that takes the
+    tuned entry.  Entries of such plans and of plans on 16-byte boundaries are kept apart."""
+    import ctypes
+    import json
+    L = _lib.load()
+    cache = tmp_path / "tune.jsonl"
+    monkeypatch.setenv("SATGB_TUNE_CACHE", str(cache))
+    g = torch.Generator(device="cpu").manual_seed(53)
+    sizes = [(201, 301), (77, 1001), (1203, 1501)]
+    xs = [torch.randint(0, 9, s, generator=g).to(t_in).to(cuda) for s in sizes]
+    live = {}
+
+    def alloc(n, ctx):
+        live[(p := torch.cuda.caching_allocator_alloc(n, cuda, torch.cuda.current_stream()))] = n
+        return p
+
+    def free(p, ctx):
+        if p:
+            del live[p]
+            torch.cuda.caching_allocator_delete(p)
+
+    def copies():
+        return [n for n in live.values() if n % 4096]  # (a workspace is whole pages)
+
+    hooks = _lib._ALLOC_FN(alloc), _lib._FREE_FN(free)
+
+    def check(plan, outs):
+        for o in outs:
+            o.view(torch.int32).zero_()
+        plan.exec()
+        plan.check()
+        for x, o in zip(xs, outs):
+            want = x.to(torch.int64).cumsum(0).cumsum(1)
+            got = o.double().to(torch.int64) if t_out == torch.float32 else o.view(torch.int32).to(torch.int64)
+            assert torch.equal(got, want)
+
+    sat_gb300.release()
+    torch.cuda.synchronize()
+    assert L.satgb_set_allocator(*hooks, None) == 0
+    try:
+        outs = [torch.empty(s, dtype=torch.int32, device=cuda).view(t_out) for s in sizes]
+        sat_gb300.set_config(first)
+        plan = sat_gb300.BatchPlan(xs, outs)
+        sat_gb300.set_config(-1)
+        tuned = plan.autotune()
+        mine = copies()
+        check(plan, outs)
+        plan.close()
+        fresh = sat_gb300.BatchPlan(xs, outs)
+        assert [c["config"] for c in fresh.classes()] == list(tuned)
+        assert copies() == mine
+        check(fresh, outs)
+        fresh.close()
+        aligned = [torch.zeros((h, 1024), dtype=t_in, device=cuda) for h, _ in sizes]
+        plan = sat_gb300.BatchPlan(aligned, [torch.empty(a.shape, dtype=torch.int32, device=cuda).view(t_out) for a in aligned])
+        plan.autotune()
+        plan.close()
+        assert not live
+    finally:
+        sat_gb300.set_config(-1)
+        torch.cuda.synchronize()
+        assert L.satgb_set_allocator(_lib._ALLOC_FN(), _lib._FREE_FN(), None) == 0
+    rows = {json.loads(line)["tma"] for line in cache.read_text().splitlines() if "batch_in" in line}
+    assert 1 in rows and any(r & 2 for r in rows)
