@@ -706,7 +706,8 @@ struct TilePlan {
 constexpr int kOrderDiag = 0;
 constexpr int kOrderRows = 1;
 
-template <bool REV, int ORDER = kOrderDiag>
+// P32: plan in 32-bit arithmetic where the tiles are few enough.
+template <bool REV, int ORDER = kOrderDiag, bool P32 = true>
 __device__ __noinline__ TilePlan plan_tile(const SatParams& P, unsigned long long tk) {
   TilePlan tp;
   tp.t = -1;
@@ -722,7 +723,7 @@ __device__ __noinline__ TilePlan plan_tile(const SatParams& P, unsigned long lon
     tp.pl = 0;
     return tp;
   }
-  if (P.n_images == 1 && P.n_tiles < kTiles32) {
+  if (P32 && P.n_images == 1 && P.n_tiles < kTiles32) {
     const uint32_t per = (uint32_t)P.img0.tiles_per_plane, q32 = (uint32_t)q;
     const int ntx = P.img0.ntx;
     const uint32_t pl = P.img0.planes > 1 ? q32 / per : 0u, k = q32 - pl * per;
@@ -796,11 +797,11 @@ __device__ __forceinline__ void issue_tile(const SatParams& P, const TilePlan& t
 // Takes ticket `tk`, maps it to a tile and starts its input on its way into
 // stage `st`.  Returns false once the tickets are exhausted (the stage then
 // carries -1).
-template <class TIn, bool REV, int TW, int TH, int STAGE_BYTES, int ORDER = kOrderDiag>
+template <class TIn, bool REV, int TW, int TH, int STAGE_BYTES, int ORDER = kOrderDiag, bool P32 = true>
 __device__ __noinline__ bool produce(const SatParams& P, unsigned long long tk, int st, TIn* stage_ptr,
                                         long long* s_tile, int* s_img, int* s_tx, int* s_ty, int* s_pl,
                                         unsigned long long* s_full) {
-  const TilePlan tp = plan_tile<REV, ORDER>(P, tk);
+  const TilePlan tp = plan_tile<REV, ORDER, P32>(P, tk);
   issue_tile<TIn, TW, TH, STAGE_BYTES>(P, tp, st, stage_ptr, s_tile, s_img, s_tx, s_ty, s_pl, s_full);
   return tp.t >= 0;
 }
@@ -866,6 +867,11 @@ __global__ void __launch_bounds__(NW * 32, MINB) sat_tile_kernel(const __grid_co
   constexpr int K = Ar<A>::K;
   constexpr bool WIDEN = !DIRECT && sizeof(TIn) < sizeof(TOut); // outputs overlap other threads' inputs in the stage
   constexpr int ORDER = KIND == kKindCols ? kOrderRows : kOrderDiag;
+  // The producer here is a thread of a compute warp that takes a ticket between two barriers.  With diagonals planned in
+  // 32 bits SATs were slower, nothing else changed (us, so and by the search: 192 planes of 1024^2 f32 438 and
+  // 407, i32 440 and 409, u8 -> u32 315 and 294; 64 planes f32 147 and 143; compensated f32 1500^2 24.1 and 22.0), column
+  // scans, which have no diagonals, faster (f32 8192^2 98.4 and 100.1).
+  constexpr bool P32 = KIND == kKindCols;
   using AR = Ar<A>;
 
   extern __shared__ __align__(128) unsigned char dsmem[];
@@ -906,7 +912,7 @@ __global__ void __launch_bounds__(NW * 32, MINB) sat_tile_kernel(const __grid_co
 #pragma unroll
     for (int s = 0; s < S - 1; ++s) {
       if (producing)
-        producing = produce<TIn, REV, TW, TH, SH::IN_BYTES, ORDER>(P, atomicAdd(&P.ws->ticket, 1ull), s,
+        producing = produce<TIn, REV, TW, TH, SH::IN_BYTES, ORDER, P32>(P, atomicAdd(&P.ws->ticket, 1ull), s,
                                                             stages + s * STAGE_ELEMS, s_tile, s_img, s_tx, s_ty,
                                                             s_pl, s_full);
     }
@@ -1166,7 +1172,7 @@ __global__ void __launch_bounds__(NW * 32, MINB) sat_tile_kernel(const __grid_co
       // tile k+S-1 into the stage whose store (tile k-1) has finished reading it
       const int ps = (st + S - 1) % S;
       bulk_wait_read_all();
-      producing = produce<TIn, REV, TW, TH, SH::IN_BYTES, ORDER>(P, pending, ps, stages + ps * STAGE_ELEMS, s_tile, s_img,
+      producing = produce<TIn, REV, TW, TH, SH::IN_BYTES, ORDER, P32>(P, pending, ps, stages + ps * STAGE_ELEMS, s_tile, s_img,
                                                           s_tx, s_ty, s_pl, s_full);
       if (producing) pending = atomicAdd(&P.ws->ticket, 1ull);
     }
