@@ -349,10 +349,11 @@ __global__ void __launch_bounds__(TileShapeWS<TIn, TOut, A, RPW, NWC, DIRECT, CT
         RowSeg<TIn, CPT> xin[RPW];
 #pragma unroll
         for (int r = 0; r < RPW; ++r) xin[r].u.v = *reinterpret_cast<const typename RowSeg<TIn, CPT>::V*>(sb + r * TW);
+        // (the tile's plane too: the producer writes the next tile's over it)
+        TOut* out = static_cast<TOut*>(D.out) + (long long)s_pl[st] * D.out_plane + (y0 + warp * RPW) * D.out_pitch + xt;
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&s_done[st]));
         const bool vout = (flags & kOutVec) && nvalid == CPT;
-        TOut* out = static_cast<TOut*>(D.out) + (long long)s_pl[st] * D.out_plane + (y0 + warp * RPW) * D.out_pitch + xt;
 #pragma unroll
         for (int i = 0; i < RPW; ++i) {
           const int r = REV ? RPW - 1 - i : i;

@@ -1031,3 +1031,23 @@ def test_autotuned_plan_is_the_plan_its_entry_makes(cuda, tmp_path, monkeypatch,
         assert L.satgb_set_allocator(_lib._ALLOC_FN(), _lib._FREE_FN(), None) == 0
     rows = {json.loads(line)["tma"] for line in cache.read_text().splitlines() if "batch_in" in line}
     assert 1 in rows and any(r & 2 for r in rows)
+
+
+@pytest.mark.parametrize("cfg", [0, 1, 2, 3, 5, 6])
+@pytest.mark.parametrize("t", [torch.int32, torch.float64])
+def test_stacks_keep_their_planes(cuda, cfg, t):
+    """Stacks of planes through every kernel, many tiles a CTA and the plane changing from one tile of a stage to the
+    next: each tile's results in its own plane, aligned and odd planes, both directions."""
+    g = torch.Generator(device=cuda).manual_seed(61)
+    try:
+        sat_gb300.set_config(cfg)
+        for n, h, w in [(700, 130, 128), (500, 127, 257), (64, 513, 387), (3, 2049, 2050)]:
+            x = torch.randint(0, 9, (n, h, w), generator=g, device=cuda, dtype=torch.int32).to(t)
+            for rev in (False, True):
+                want = (x.flip((1, 2)) if rev else x).cumsum(1, dtype=t).cumsum(2, dtype=t)
+                want = want.flip((1, 2)) if rev else want
+                for _ in range(3):
+                    assert torch.equal(sat_gb300.sat(x, t, reverse=rev), want), (n, h, w, rev)
+        sat_gb300.stream_check()
+    finally:
+        sat_gb300.set_config(-1)
