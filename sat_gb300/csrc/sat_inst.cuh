@@ -122,7 +122,7 @@ Variant make_variant_ws(int in_t, int out_t, int mode, int cfg) {
                  SH::TH, SH::TW, Ar<A>::K, SH::THREADS, SH::DYN_SMEM};
 }
 
-// The same three for sat_tile_kernel_wd (1-byte inputs, 4-byte sums).
+// The same three for sat_tile_kernel_wd (1- and 4-byte inputs, 4-byte sums).
 template <class TIn, class TOut, class A, bool REV, bool SKEW>
 cudaError_t prepare_one_wd() {
   return cudaFuncSetAttribute(&sat_tile_kernel_wd<TIn, TOut, A, REV, SKEW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -154,7 +154,7 @@ cudaError_t launch_impl_wd(const SatParams& p, int grid, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-// Configuration 5: the packed kernel for 1-byte inputs with 4-byte sums, sat_tile_kernel_ws with direct
+// Configuration 5: the deep kernel for 1- and 4-byte inputs with 4-byte sums, sat_tile_kernel_ws with direct
 // stores for every other accumulator.
 template <class TIn, class TOut, class A, bool REV>
 Variant make_variant_5(int in_t, int out_t, int mode) {
@@ -225,9 +225,10 @@ Variant make_variant_rm(int in_t, int out_t, int mode, int cfg) {
 //      the compensated f32 SAT measured 0.284 ms with 64-row and 0.217 ms with
 //      128-row tiles at 8192^2)
 //   4: (1-byte inputs, 4-byte sums only, SG_TALL) pipelined, 256-row tiles, direct stores
-//   5: warp-specialized with direct stores, 8 rows a compute warp: 128-row
-//      tiles and 16 compute warps for 4-byte accumulators (64-row tiles and 8
-//      compute warps for 8-byte ones)
+//   5: warp-specialized with direct stores, 8 rows a compute warp: for 4-byte
+//      accumulators the deep kernel (128-row tiles for 1-byte, 96-row tiles for
+//      4-byte inputs, which SG_WIDE gives a second kernel with 128-row tiles); 64-row
+//      tiles and 8 compute warps for 8-byte accumulators
 //   6: as 5, with the tiles in row-major order: rowleft is the sum of every
 //      row aggregate to the left, the look-back is vertical only (no corner)
 #define SG_CFG1_RPW(A) (sizeof(A) == 8 ? 4 : 8)
@@ -255,6 +256,12 @@ Variant make_variant_rm(int in_t, int out_t, int mode, int cfg) {
 #define SG_TALL(TIN, TOUT, A, IT, OT)                                                      \
   satgb::make_variant<TIN, TOUT, A, false, 16, 16, 1, satgb::kKindSat, true>(IT, OT, 0, 4), \
       satgb::make_variant<TIN, TOUT, A, true, 16, 16, 1, satgb::kKindSat, true>(IT, OT, 0, 4)
+
+// configuration 5's second kernel for 4-byte inputs with 4-byte sums: sat_tile_kernel_ws with direct
+// stores and 128-row tiles
+#define SG_WIDE(TIN, TOUT, A, IT, OT)                                                              \
+  satgb::make_variant_ws<TIN, TOUT, A, false, 8, 16, true>(IT, OT, 0, satgb::kConfig5Wide), \
+      satgb::make_variant_ws<TIN, TOUT, A, true, 8, 16, true>(IT, OT, 0, satgb::kConfig5Wide)
 
 #define SG_TABLE(NAME, ...)                                   \
   namespace satgb {                                           \

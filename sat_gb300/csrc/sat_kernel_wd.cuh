@@ -145,12 +145,6 @@ __device__ __forceinline__ A row_totals(const A (&v)[8], int lane) {
   return AR::add(t, __shfl_xor_sync(0xffffffffu, t, 1));
 }
 
-// The corner's sums: one value a tile, whose chain down the image is the longest and enters every
-// result, so f32 sums are kept in f64 there (f32 8192^2: mean relative
-// error 8.5e-8 with the chain in f32, 5.7e-8).
-template <class A>
-using CornerAcc = std::conditional_t<sizeof(A) == 4 && (A(0.5f) != A(0)), double, A>;
-
 // The sum of a word's four pixels picked by the mask's bytes (0 or 1), plus c.
 template <class TIn>
 __device__ __forceinline__ uint32_t pixel_sum(uint32_t w, uint32_t mask, uint32_t c) {

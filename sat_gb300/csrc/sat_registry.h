@@ -35,6 +35,8 @@ struct TileConfig {
   const char* name;
 };
 constexpr int kNumConfigs = 7;
+// The second kernel of configuration 5 for 4-byte inputs (config5_kernel in satgb_api.cu): no configuration of its own.
+constexpr int kConfig5Wide = kNumConfigs;
 extern const TileConfig kConfigs[kNumConfigs];
 
 // Lists of variants, one per instantiation translation unit.

@@ -263,7 +263,7 @@ Layout layout_for(long long n_tiles, const Variant* v) {
   L.row_off = sizeof(WsHeader);
   L.col_off = L.row_off + (size_t)n_tiles * v->TH * v->K * w;
   L.corner_off = L.col_off + (size_t)n_tiles * v->TW * v->K * w;
-  L.total = L.corner_off + (size_t)n_tiles * std::max(v->K, 2) * w; // (configuration 5 keeps f32 corners in f64)
+  L.total = L.corner_off + (size_t)n_tiles * std::max(v->K, 2) * w; // (the warp-specialized kernels keep f32 corners in f64)
   return L;
 }
 
@@ -596,6 +596,28 @@ int choose_config_locked(int in_t, int out_t, int mode, int dir, long long w, lo
                         planes, off16);
 }
 
+// Configuration 5 of 4-byte inputs with 4-byte sums is one of two kernels: the deep one (sat_kernel_wd.cuh), whose carries
+// have two tile periods, and 128-row tiles (sat_kernel_ws.cuh), which have one, but a quarter fewer tiles.
+// - Rows that TMA cannot address, neither one by one nor in groups: 128 rows (us, deep and 128-row: views of
+//   8192 rows of 8187 f32 231 and 208, i32 230 and 201; 3 planes of 4095^2 f32 158 and 147; 8 of them 412 and 373).
+// - f32 where an anti-diagonal has work for enough CTAs that look-backs find their sums published: 128 rows from
+//   0.4 tiles of 128 x 128 a diagonal and SM in one image (16384^2, 64 tiles, 399 and 394; 20480^2 604 and 585; at 56
+//   tiles 14336^2 311 and 311; below 12288^2, 48 tiles, 234 and 238, 8192^2 114.2 and 115.2, 1024 x 65536 141 and 194),
+//   from 0.26 over the images of a plan, whose chains are shorter (64 of 1024^2, 273 tiles, 109 and 95, 512 of sides
+//   64..4096 865 and 791; at 40 tiles 20 of them 77.2 and 74.0; below 4 of 2048^2, 33 tiles, 38.4 and 38.6).  Integers
+//   stay on the deep kernel (i32 16384^2 394 and 459, 512 of sides 64..4096 877 and 900), and so do packed rows in
+//   groups (8191^2 f32 143 and 191; in plans up to an eighth of the pixels is cheaper copied: 16 images of
+//   2048^2, 2 of them packed, 120.4 and 120.0, 4 of them 126 and 134).
+// diagonal: tiles of 128 x 128 on an anti-diagonal in the mean; groups: enough rows come in groups.
+const Variant* config5_kernel(const Variant* v, double diagonal, bool plan, int sms, bool plain_rows, bool groups) {
+  if (!v || v->cfg != 5) return v;
+  const bool wide = plain_rows || (v->in_t == SATGB_F32 && !groups && diagonal >= (plan ? 0.26 : 0.4) * sms);
+  const Variant* w = wide ? find_variant(v->in_t, v->out_t, v->mode, v->dir, kConfig5Wide) : nullptr;
+  return w ? w : v;
+}
+
+int config_of(const Variant* v) { return v->cfg == kConfig5Wide ? 5 : v->cfg; }
+
 satgb_status launch_locked(const Variant* v, const ImageDesc* table_dev, const ImageDesc& img0,
                            long long n_images, long long n_tiles, Workspace& ws, int dev,
                            cudaStream_t s, const ulonglong2* order = nullptr, bool skewed = false) {
@@ -699,6 +721,12 @@ satgb_status sat_single(int in_t, int out_t, int mode, int dir, const void* d_in
                      default_config(width, height, sms_of(dev), (int)in_sz, (int)out_sz,
                                     mode == SATGB_MODE_COMPENSATED, planes, off16));
   if (!v) v = find_variant(in_t, out_t, mode, dir, 0);
+  if (v && v->cfg == 5) {
+    const double ntx = (double)((width + 127) / 128), nty = (double)((height + 127) / 128);
+    const bool groups = skew_rows(v, d_in, in_pitch, width, height, planes, in_sz) != 0;
+    const bool tma = tma_ok(d_in, width, height, in_pitch, planes, planes > 1 ? in_plane : 0, in_sz);
+    v = config5_kernel(v, ntx * nty / (ntx + nty - 1), false, sms_of(dev), in_sz == 4 && !tma && !groups, groups);
+  }
   if (!v) return fail(SATGB_ERR_UNSUPPORTED_TYPES, "no kernel for %s -> %s mode %d dir %d", dtype_name(in_t), dtype_name(out_t), mode, dir);
   Workspace& ws = g_ws[std::make_pair(dev, (void*)s)];
   // A large image of 1-byte inputs whose rows TMA cannot address (packed rows
@@ -1176,7 +1204,16 @@ const Variant* seg_variant(const satgb_batch_plan_s* p, int cls, int cfg) {
   const Variant* v = find_variant(p->in_t, p->out_t, p->mode, p->dir, cfg);
   if (!v) v = find_variant(p->in_t, p->out_t, p->mode, p->dir, batch_default_config(p, cls));
   if (!v) v = find_variant(p->in_t, p->out_t, p->mode, p->dir, 0);
-  return v;
+  if (!v || v->cfg != 5) return v;
+  double tiles = 0, diagonals = 1, grouped = 0;
+  for (const ImgCheck& c : p->seg[cls].imgs) {
+    const double ntx = (double)((c.width + 127) / 128), nty = (double)((c.height + 127) / 128);
+    tiles += ntx * nty;
+    diagonals = std::max(diagonals, ntx + nty - 1);
+    if (skew_rows(v, c.in, c.in_pitch, c.width, c.height, 1, dtype_size(p->in_t)))
+      grouped += (double)c.width * (double)c.height;
+  }
+  return config5_kernel(v, tiles / diagonals, true, sms_of(p->dev), false, grouped > 0.125 * p->seg[cls].pixels);
 }
 
 // (Re)builds a class's descriptor table for the kernel `v`; called with g_mu
@@ -1509,8 +1546,8 @@ satgb_status satgb_batch_plan_autotune(satgb_batch_plan* p, satgb_stream stream,
     float best_ms = 1e30f;
     for (int cfg = 0; cfg < kNumConfigs && st == SATGB_OK; ++cfg) {
       const Variant* only[kBatchClasses] = {};
-      only[cls] = find_variant(p->in_t, p->out_t, p->mode, p->dir, cfg);
-      if (!only[cls]) continue;
+      if (!find_variant(p->in_t, p->out_t, p->mode, p->dir, cfg)) continue;
+      only[cls] = seg_variant(p, cls, cfg);
       st = plan_layout(p, only, s);
       if (st == SATGB_OK) st = plan_time(p, s, e0, e1, &ms);
       if (st == SATGB_OK && ms < best_ms) {
@@ -1543,8 +1580,8 @@ satgb_status satgb_batch_plan_autotune(satgb_batch_plan* p, satgb_stream stream,
   if (st == SATGB_OK) {
     for (int cls = 0; cls < kBatchClasses; ++cls) {
       if (!best[cls]) continue;
-      g_batch_tune[batch_key(p, cls, sms)] = best[cls]->cfg;
-      if (configs) configs[cls] = best[cls]->cfg;
+      g_batch_tune[batch_key(p, cls, sms)] = config_of(best[cls]);
+      if (configs) configs[cls] = config_of(best[cls]);
     }
     tune_save_locked();
     return p->n_tiles > 0 ? plan_capture(p) : SATGB_OK;
@@ -1579,7 +1616,7 @@ satgb_status satgb_batch_plan_info(const satgb_batch_plan* p, int64_t* n_tiles, 
   if (n_tiles) *n_tiles = p->n_tiles;
   if (config) {
     // the configuration of the large class, or of the small one if it is alone
-    *config = p->seg[0].n_images ? p->seg[0].v->cfg : (p->seg[1].n_images ? p->seg[1].v->cfg : -1);
+    *config = p->seg[0].n_images ? config_of(p->seg[0].v) : (p->seg[1].n_images ? config_of(p->seg[1].v) : -1);
   }
   return SATGB_OK;
 }
@@ -1590,7 +1627,7 @@ satgb_status satgb_batch_plan_classes(const satgb_batch_plan* p, int64_t* n_imag
     const BatchSeg& g = p->seg[cls];
     if (n_images) n_images[cls] = g.n_images;
     if (n_tiles) n_tiles[cls] = g.n_tiles;
-    if (configs) configs[cls] = g.n_images ? g.v->cfg : -1;
+    if (configs) configs[cls] = g.n_images ? config_of(g.v) : -1;
   }
   return SATGB_OK;
 }

@@ -1051,3 +1051,51 @@ def test_stacks_keep_their_planes(cuda, cfg, t):
         sat_gb300.stream_check()
     finally:
         sat_gb300.set_config(-1)
+
+
+@pytest.mark.parametrize("t", [torch.float32, torch.int32, torch.uint32])
+def test_both_kernels_of_configuration_5(cuda, t):
+    """4-byte images on both sides of the choice between the deep kernel and 128-row tiles: views whose rows TMA cannot
+    address, stacks of odd planes, an image of long anti-diagonals, plans with many tiles a diagonal, with a few packed images
+    among aligned ones and with many, both directions.  Sums below 2^24: f32 is exact."""
+    g = torch.Generator(device=cuda).manual_seed(59)
+    bits = torch.int32 if t == torch.uint32 else t
+
+    def image(*shape):
+        return (torch.rand(shape, generator=g, device=cuda) < 0.05).to(bits)
+
+    def want(x, rev):
+        y = x.to(torch.int32)
+        y = y.flip((-2, -1)) if rev else y
+        y = y.cumsum(-2).cumsum(-1).to(bits)
+        return y.flip((-2, -1)) if rev else y
+
+    try:
+        for rev in (False, True):
+            for cfg, (h, w, off, pad) in [(5, (130, 200, 1, 3)), (5, (97, 129, 2, 1)), (5, (1, 1, 1, 4)), (5, (300, 2, 1, 2)),
+                                          (-1, (3000, 2999, 1, 3)), (-1, (2500, 3101, 3, 2))]:
+                sat_gb300.set_config(cfg)
+                x = image(h, w + off + pad)[:, off:off + w]
+                out = torch.full((h, w + pad), 7, dtype=bits, device=cuda)
+                sat_gb300.sat(x.view(t), t, reverse=rev, out=out[:, :w].view(t))
+                assert torch.equal(out[:, :w], want(x, rev)), (h, w, rev)
+                assert bool((out[:, w:] == 7).all())
+            sat_gb300.set_config(-1)
+            x = image(2, 3071, 3073)
+            assert torch.equal(sat_gb300.sat(x.view(t), t, reverse=rev).view(bits), want(x, rev)), rev
+            x = image(16000, 16000)
+            assert torch.equal(sat_gb300.sat(x.view(t), t, reverse=rev).view(bits), want(x, rev)), rev
+            del x
+            for packed in (0, 1, 2, 3, 16):
+                xs = [image(1023, 1021 if i < packed else 1024) for i in range(16)] + [image(1100, 900)[:, 1:850]]
+                outs = [torch.empty(x.shape, dtype=bits, device=cuda) for x in xs]
+                plan = sat_gb300.BatchPlan([x.view(t) for x in xs], [o.view(t) for o in outs], reverse=rev)
+                assert plan.classes()[0]["config"] == 5
+                plan.exec()
+                plan.check()
+                for i, (x, out) in enumerate(zip(xs, outs)):
+                    assert torch.equal(out, want(x, rev)), (packed, i, rev)
+                plan.close()
+        sat_gb300.stream_check()
+    finally:
+        sat_gb300.set_config(-1)
