@@ -203,6 +203,9 @@ satgb_status satgb_box_filter_fwd(const satgb_box_desc* desc, satgb_stream strea
  * The means may not overlap the image. */
 satgb_status satgb_box_filter_fwd_x(const satgb_box_desc* desc, const void* d_x, int64_t x_pitch,
                                     int64_t x_plane_stride, satgb_stream stream);
+/* 1 where satgb_box_filter_fwd_x would use a scratch SAT if it had one (d_sat,
+ * its pitch and plane stride are not looked at), 0 where it would not. */
+int satgb_box_filter_fwd_x_scratch(const satgb_box_desc* desc);
 /* The adjoint of satgb_box_filter_fwd: dL/dSAT from the gradients of all the
  * radii's means (the four-corner scatter, computed as a gather so it is
  * deterministic).  d_sat is overwritten. */

@@ -272,11 +272,6 @@ def box_means_from_sat(sat_t: torch.Tensor, radii: Sequence[int], out=None, stre
     return out
 
 
-# Radii from which the library may go through a SAT (box_fused.cu: two radii of 34 leave an SM two
-# blocks); up to there a scratch SAT would be allocated for nothing.
-_SCRATCH_RADIUS = 34
-
-
 def box_means(x: torch.Tensor, radii: Sequence[int], out=None, stream=None) -> torch.Tensor:
     """Clipped box means of every radius of the image x itself: (..., H, W) ->
     (..., R, H, W), in one launch, or for large radii, where that is faster, through
@@ -287,7 +282,8 @@ def box_means(x: torch.Tensor, radii: Sequence[int], out=None, stream=None) -> t
     dx, pitch, plane = d.d_sat, d.sat_pitch, d.sat_plane_stride
     d.d_sat = None
     fwd, handle, scratch = _lib.load().satgb_box_filter_fwd_x, _call_stream(stream), None
-    if min(max(d.radius), max(d.width, d.height) - 1) >= _SCRATCH_RADIUS:
+    # (up to radius 15 the library never takes it)
+    if max(d.radius) > 15 and _lib.load().satgb_box_filter_fwd_x_scratch(ctypes.byref(d)):
         # from the pool of the stream that uses it: the block goes back, and to its next owner, in that
         # stream's order, whatever stream is current
         scratch = torch.cuda.caching_allocator_alloc(4 * x.numel(), x.device, handle)

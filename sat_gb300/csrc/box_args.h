@@ -31,9 +31,9 @@ satgb_status box_check_desc(const satgb_box_desc* d, BoxArgs& a);
 // their gradient with respect to the image straight from the means' gradients
 // (`a.sat` is the gradient written), each in one launch.  *done is false, and
 // nothing was launched, when the radii are too large for the kernels' shared
-// memory or, for the means unless `only_way`, going through the SAT is faster: the
-// caller then does that.
-satgb_status box_means_fused(const BoxArgs& a, cudaStream_t s, bool only_way, bool* done);
+// memory or, unless `only_way`, going through the SAT is faster: the
+// caller then does that.  launch false: only *done.
+satgb_status box_means_fused(const BoxArgs& a, cudaStream_t s, bool only_way, bool launch, bool* done);
 satgb_status box_grad_fused(const BoxArgs& a, cudaStream_t s, bool* done);
 
 }  // namespace satgb

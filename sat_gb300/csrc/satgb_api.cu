@@ -1050,6 +1050,17 @@ satgb_status satgb_autotune(satgb_dtype in_t, satgb_dtype out_t, int mode, const
 // ---------------------------------------------------------------------------
 // box-filter backward to the image
 // ---------------------------------------------------------------------------
+int satgb_box_filter_fwd_x_scratch(const satgb_box_desc* desc) {
+  satgb::BoxArgs a;
+  if (!desc) return 0;
+  satgb_box_desc d = *desc;
+  if (!d.d_sat) d.d_sat = d.d_box[0], d.sat_pitch = d.box_pitch, d.sat_plane_stride = d.box_plane_stride;
+  if (satgb::box_check_desc(&d, a) != SATGB_OK || d.width == 0 || d.height == 0 || d.n_planes == 0) return 0;
+  bool one = false;
+  satgb::box_means_fused(a, nullptr, false, false, &one);
+  return one ? 0 : 1;
+}
+
 satgb_status satgb_box_filter_fwd_x(const satgb_box_desc* desc, const void* d_x, int64_t x_pitch,
                                     int64_t x_plane_stride, satgb_stream stream) {
   if (!desc) return fail(SATGB_ERR_INVALID_ARG, "box means: null descriptor");
@@ -1071,7 +1082,7 @@ satgb_status satgb_box_filter_fwd_x(const satgb_box_desc* desc, const void* d_x,
       return fail(SATGB_ERR_INVALID_ARG, "box means: the means overlap the image");
   }
   bool done = false;
-  st = satgb::box_means_fused(a, (cudaStream_t)stream, !desc->d_sat, &done);
+  st = satgb::box_means_fused(a, (cudaStream_t)stream, !desc->d_sat, true, &done);
   if (st != SATGB_OK || done) return st;
   if (!desc->d_sat)
     return fail(SATGB_ERR_NOT_FOUND, "box means: radii above 64 need a scratch SAT (descriptor's d_sat)");

@@ -462,3 +462,41 @@ def test_box_layer_infinities_spoil_no_more_than_the_sat_path(cuda, shape, radii
             assert not bool(dx[0][holds].isfinite().any()), (r0, c0, r)
         for i in range(1, shape[0]):
             assert bool(m[i].isfinite().all()) and bool(dx[i].isfinite().all())
+
+
+@pytest.mark.parametrize("shape,radii,scratch", [
+    ((4, 64, 16), (15,), 0), ((4, 64, 16), (16,), 1), ((4, 64, 33), (23,), 0), ((4, 64, 33), (24,), 1),   # narrow planes
+    ((4, 64, 64), (30,), 0), ((4, 64, 64), (31,), 1), ((4, 64, 128), (23, 60), 1),
+    ((2, 300, 300), (27,), 0), ((2, 300, 300), (3, 31), 0), ((2, 300, 300), (34,), 0), ((2, 300, 300), (35,), 1),  # few blocks
+    ((600, 256, 256), (27,), 0), ((600, 256, 256), (28,), 1), ((600, 256, 258), (31,), 0), ((600, 256, 258), (32,), 1),
+    ((900, 160, 160), (34,), 0), ((300, 256, 256), (3, 31), 0), ((300, 256, 256), (3, 32), 1),
+    ((300, 100, 128), (3, 5, 17, 32), 0), ((300, 100, 256), (3, 5, 17, 40), 1), ((60, 100, 1000), (3, 5, 17, 46), 1),
+])
+def test_box_layer_both_ways(cuda, shape, radii, scratch):
+    """Means and gradient on both sides of the choice between one launch and the way through the SAT: plane widths,
+    radii, numbers of blocks.  Bounds: window_error, and through the SAT 4 roundings of its largest value over the smallest
+    window, for the gradient 8 of the sum of all 4 |g| / area."""
+    g = torch.Generator(device=cuda).manual_seed(67)
+    x = torch.randn(shape, generator=g, device=cuda)
+    w = torch.randn(shape[:1] + (len(radii),) + shape[1:], generator=g, device=cuda)
+    out = torch.empty_like(w)
+    import ctypes
+    assert sat_gb300._lib.load().satgb_box_filter_fwd_x_scratch(ctypes.byref(api._box_desc(x, out, radii))) == scratch
+    api.box_means(x, radii, out=out)
+    dx = api.box_means_grad_x(w, radii)
+    H, W = shape[-2:]
+    dtol = 0.0
+    for n in (0, shape[0] // 2, shape[0] - 1):
+        x64 = x[n].double().requires_grad_(True)
+        m64 = box_means64(x64, radii)
+        (dx64,) = torch.autograd.grad(m64, x64, w[n].double())
+        smax = float(sat64(x[n]).abs().max())
+        dtol = 0.0
+        for k, r in enumerate(radii):
+            area = (min(r, H - 1) + 1) * (min(r, W - 1) + 1)
+            tol = window_error(min(r, max(H, W) - 1)) + 4 * EPS32 * smax / area + 1e-7
+            err = float((out[n, k].double() - m64[k]).abs().max())
+            assert err <= tol, (n, r, err, tol)
+            dtol += window_error(min(r, max(H, W) - 1)) + 8 * EPS32 * 4 * float(w[n, k].abs().sum()) / area
+        err = float((dx[n].double() - dx64).abs().max())
+        assert err <= dtol, (n, err, dtol)
