@@ -870,8 +870,9 @@ __global__ void __launch_bounds__(NW * 32, MINB) sat_tile_kernel(const __grid_co
   // The producer here is a thread of a compute warp that takes a ticket between two barriers.  With diagonals planned in
   // 32 bits SATs were slower, nothing else changed (us, so and by the search: 192 planes of 1024^2 f32 438 and
   // 407, i32 440 and 409, u8 -> u32 315 and 294; 64 planes f32 147 and 143; compensated f32 1500^2 24.1 and 22.0), column
-  // scans, which have no diagonals, faster (f32 8192^2 98.4 and 100.1).
-  constexpr bool P32 = KIND == kKindCols;
+  // scans of 4-byte sums, which have no diagonals, faster (f32 8192^2 98.4 and 100.1), of f64 sums some of both (u8 -> f64
+  // 1024^2 31.4 and 25.9, 64 x 500 13.8 and 15.5).
+  constexpr bool P32 = KIND == kKindCols && sizeof(A) == 4;
   using AR = Ar<A>;
 
   extern __shared__ __align__(128) unsigned char dsmem[];
