@@ -6,15 +6,15 @@
 // rows go through registers: a warp sums its R rows (a lane a column, rows of the strip 32 coalesced
 // elements at any alignment), the warps' sums meet in shared memory, and each warp runs down its rows from the
 // sum of everything above.  The next block's loads are in flight meanwhile (two blocks ahead f32 4096^2 was 26.6 us
-// for 28.5, but 4600 x 3000 30.3 for 25.9: 64 registers a thread are short).
+// for 28.5, but 4600 x 3000 30.3 for 25.9: 64 registers a thread were short).
 //
 // What bounds it: a block's time on one SM, whose stores (25 bytes a cycle at most) and whose
-// scan over the warps follow one another (1.35 us a block of 256 rows of 4-byte results, half of it the
-// stores); f64 results the FP64 adds, 7 us.  Memory only where every SM has a strip.  With 16 warps of 16
-// rows and each warp adding up the ones before it a block took 2 us, and f32 errors doubled; an f32
+// scan over the warps follow one another (1.1 us a block of 256 rows of 4-byte results, half of it the
+// stores); f64 results the FP64 adds, 7 us (9 from narrower inputs).  Memory only where every SM has a strip.  With 16
+// warps of 16 rows and each warp adding up the ones before it a block took 2 us, and f32 errors doubled; an f32
 // column's sum over the blocks is a two-sum pair (mean relative error at 8192 rows 7.9e-8 -> 4.6e-8).
-// us, before (look-back over tiles) and now: f32 256 x 256 7.9 -> 3.4, 1024^2 10.4 -> 7.1, 4096 x 1000 13.3 -> 8.3,
-// 4096^2 33.8 -> 29, packed 3001 x 3000 32.8 -> 25.1, packed 8191^2 221 -> 146; f64 4096^2 176 -> 117.
+// us in a graph, look-back over tiles and strips: f32 256 x 256 8.0 and 3.1, 1024^2 10.1 and 6.2, 4096 x 2048 18.1 and
+// 11.1, 4096^2 33.6 and 28.7, packed 3001 x 3003 33.4 and 17.6, 8191^2 220 and 143; f64 4096^2 177 and 116.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -54,6 +54,12 @@ struct Carry<float> {
   }
 };
 
+template <class T>
+__device__ __forceinline__ T* next_row(T* p, long long pitch) {
+  asm volatile("" : "+l"(p));
+  return p + pitch;
+}
+
 template <class TIn, class TOut, class A>
 __global__ void __launch_bounds__(kColWarps * 32, 1)
     scan_cols_strip_kernel(const TIn* in, long long in_pitch, TOut* out, long long out_pitch, long long width,
@@ -62,20 +68,24 @@ __global__ void __launch_bounds__(kColWarps * 32, 1)
   using AR = Ar<A>;
   __shared__ A s_sum[NW][33]; // a warp's sums by column, then the sums of the warps above (and of all blocks above)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const long long col = (long long)blockIdx.x * 32 + lane;
-  const bool valid = col < width;
-  const long long n_blocks = (height + BLOCK - 1) / BLOCK, full = valid ? height / BLOCK : 0;
+  // Lanes past the last column compute and store that column too, the same bits to the same place, so that all lanes go one
+  // way (with lanes that did nothing the last strip's CTA went two, took half as long again, and the launch with it).
+  const long long mine = (long long)blockIdx.x * 32 + lane, col = mine < width ? mine : width - 1;
+  const long long n_blocks = (height + BLOCK - 1) / BLOCK, full = height / BLOCK;
   const TIn* gin = in + (long long)warp * R * in_pitch + col; // the warp's rows of the next block to load
   TOut* gout = out + (long long)warp * R * out_pitch + col;   // ... to store
 
+  // A row after the other from one pointer: the pitch's multiples, which the compiler would otherwise keep
+  // through the loop, take the registers that the rows need.
   auto load = [&](TIn (&v)[R], long long b) {
+    const TIn* p = gin;
     if (b < full) {
 #pragma unroll
-      for (int r = 0; r < R; ++r) v[r] = __ldcs(gin + r * in_pitch);
+      for (int r = 0; r < R; ++r, p = next_row(p, in_pitch)) v[r] = __ldcs(p);
     } else {
       const long long y = b * BLOCK + warp * R;
 #pragma unroll
-      for (int r = 0; r < R; ++r) v[r] = (valid && y + r < height) ? __ldcs(gin + r * in_pitch) : TIn(0);
+      for (int r = 0; r < R; ++r, p = next_row(p, in_pitch)) v[r] = y + r < height ? __ldcs(p) : TIn(0);
     }
     gin += BLOCK * in_pitch;
   };
@@ -100,18 +110,19 @@ __global__ void __launch_bounds__(kColWarps * 32, 1)
     }
     __syncthreads();
     A above = s_sum[warp][lane];
+    TOut* p = gout;
     if (b < full) {
 #pragma unroll
-      for (int r = 0; r < R; ++r) {
+      for (int r = 0; r < R; ++r, p = next_row(p, out_pitch)) {
         above = AddIn<A, TIn>::add(above, v[r]);
-        __stcs(gout + r * out_pitch, OutCvt<TOut, A>::out(above));
+        __stcs(p, OutCvt<TOut, A>::out(above));
       }
     } else {
       const long long y = b * BLOCK + warp * R;
 #pragma unroll
-      for (int r = 0; r < R; ++r) {
+      for (int r = 0; r < R; ++r, p = next_row(p, out_pitch)) {
         above = AddIn<A, TIn>::add(above, v[r]);
-        if (valid && y + r < height) __stcs(gout + r * out_pitch, OutCvt<TOut, A>::out(above));
+        if (y + r < height) __stcs(p, OutCvt<TOut, A>::out(above));
       }
     }
     gout += BLOCK * out_pitch;
@@ -138,24 +149,36 @@ cudaError_t launch_cols(const void* in, int64_t in_pitch, void* out, int64_t out
 
 }  // namespace
 
-// Strips or tiles with look-back (sat_kernel.cuh), whichever two lines through the measured times say is
-// faster.  Strips: 3 us and 1.4 a block of a strip (f64 results 7) for each wave of strips over the SMs, a third more
-// where rows are off 16-byte boundaries, and no faster than 4.7 TB/s.  Tiles: 8 us and 5.3 TB/s (f64 10 us and
-// 1.6), 3.0 where rows cannot go through TMA.  Few strips or many rows are the tiles': f32 1024 x 8192 (w x h)
-// 19 us by tiles, 46 by strips, 8192^2 100 and 116; wide and low, or packed, the strips': 8192 x 300 11.5 and 9.1.
+// Strips or tiles with look-back (sat_kernel.cuh), whichever two lines through the measured times say is faster (64
+// to 20000 columns by 64 to 8192 rows of every type, packed and padded, both ways forced: 0.2 % above the faster
+// one in the mean).  Tiles: a start and a rate in bytes in and out.  Strips: a start, and for each wave of strips over the
+// SMs another and a time a block of rows, longer where 32 results lie across 128-byte lines; no faster than 4.6
+// TB/s, 3.6 across lines.  Few strips or many rows are the tiles': f32 1024 x 8192 (w x h) 19 us by tiles, 36 by strips,
+// 8192^2 99 and 120; the strips': f32 1024 x 1000 9.9 and 6.2, 3000 x 2000 15.7 and 10.5, 4096^2 33.3 and 29.1, packed
+// 8191^2 220 and 143, f64 4096^2 177 and 116.
+struct ColsLine {
+  double tile_start, tile_rate; // us, TB/s
+  double start, wave, block;    // us: strips, a wave of them, a block of rows
+};
+
 bool scan_cols_by_strips(const void* in, int64_t in_pitch, size_t in_sz, const void* out, int64_t out_pitch,
                          size_t out_sz, int64_t width, int64_t height, int sms) {
   const int64_t strips = (width + 31) / 32;
   if (strips >= (1LL << 31) || sms < 1) return false;
-  const bool aligned = (uintptr_t)in % 16 == 0 && (uintptr_t)out % 16 == 0 && ((size_t)in_pitch * in_sz) % 16 == 0 &&
-                       ((size_t)out_pitch * out_sz) % 16 == 0;
+  const bool tma = (uintptr_t)in % 16 == 0 && (uintptr_t)out % 16 == 0 && ((size_t)in_pitch * in_sz) % 16 == 0 &&
+                   ((size_t)out_pitch * out_sz) % 16 == 0;
+  const bool lines = (uintptr_t)out % 128 == 0 && ((size_t)out_pitch * out_sz) % 128 == 0;
+  ColsLine c;
+  if (out_sz == 4 && in_sz == 1) c = {tma ? 10.8 : 13.0, tma ? 4.8 : 2.9, 0.4, 1.1, lines ? 1.42 : 1.52};
+  else if (out_sz == 4) c = {tma ? 10.0 : 11.0, tma ? 6.0 : 3.0, 0.6, 1.1, lines ? 1.2 : 1.28};
+  else if (in_sz == 1) c = {tma ? 11.9 : 12.4, tma ? 0.61 : 0.60, 1.1, 1.1, 8.9};
+  else if (in_sz == 4) c = {tma ? 11.7 : 12.4, tma ? 0.81 : 0.64, 1.1, 1.1, 8.9};
+  else c = {tma ? 10.2 : 10.9, tma ? 1.52 : 1.16, 1.0, 1.1, 6.9};
   const double blocks = (double)((height + kColWarps * kColRows - 1) / (kColWarps * kColRows));
   const double waves = (double)((strips + sms - 1) / sms);
   const double mb = (double)width * (double)height * (double)(in_sz + out_sz) * 1e-6; // a us at 1 TB/s
-  const double block = (out_sz == 8 ? 7.0 : 1.4) * (aligned ? 1.0 : 1.35);
-  const double by_strips = 3.0 + std::max(blocks * waves * block, mb / 4.7);
-  const double by_tiles = out_sz == 8 ? 10.0 + mb / 1.6 : 8.0 + mb / (aligned ? 5.3 : 3.0);
-  return by_strips < by_tiles;
+  const double by_strips = c.start + std::max(waves * (c.wave + blocks * c.block), mb / (lines ? 4.6 : 3.6));
+  return by_strips < c.tile_start + mb / c.tile_rate;
 }
 
 satgb_status scan_cols_strips(int in_t, int out_t, const void* d_in, int64_t in_pitch, void* d_out, int64_t out_pitch,
