@@ -1262,19 +1262,6 @@ satgb_status seg_build(satgb_batch_plan_s* p, BatchSeg& g, const Variant* v, cud
   return SATGB_OK;
 }
 
-// One table for both classes where they run the same kernel; called once every class has its own.
-satgb_status plan_merge(satgb_batch_plan_s* p, cudaStream_t s) {
-  seg_free(p->all);
-  p->all = BatchSeg();
-  for (auto& g : p->seg)
-    if (!g.n_tiles || g.v != p->seg[0].v) return SATGB_OK;
-  for (auto& g : p->seg) {
-    p->all.src.insert(p->all.src.end(), g.src.begin(), g.src.end());
-    p->all.n_images += g.n_images;
-  }
-  return seg_build(p, p->all, p->seg[0].v, s);
-}
-
 satgb_status plan_ws(satgb_batch_plan_s* p, cudaStream_t s) {
   size_t need = p->all.n_tiles ? layout_for(p->all.n_tiles, p->all.v).total : 0;
   p->n_tiles = 0;
@@ -1426,20 +1413,28 @@ satgb_status plan_stage_inputs(satgb_batch_plan_s* p, const Variant* const (&vs)
   return SATGB_OK;
 }
 
-// Lays the plan out for its classes' kernels (nullptr: the class stays out): staged inputs, tables,
-// workspace.  Called with g_mu held.
+// Lays the plan out for its classes' kernels (nullptr: the class stays out): staged inputs, tables (one of both
+// classes where they run the same kernel), workspace.  Called with g_mu held.
 satgb_status plan_layout(satgb_batch_plan_s* p, const Variant* const (&vs)[kBatchClasses], cudaStream_t s) {
   satgb_status st = plan_stage_inputs(p, vs, dtype_size(p->in_t), s);
+  seg_free(p->all);
+  p->all = BatchSeg();
+  const Variant* both = vs[0] == vs[1] ? vs[0] : nullptr;
   for (int cls = 0; cls < kBatchClasses && st == SATGB_OK; ++cls) {
     BatchSeg& g = p->seg[cls];
-    if (vs[cls]) {
+    seg_free(g);
+    g.n_tiles = 0;
+    if (both) {
+      g.v = both;
+      for (const ImgCheck& c : g.src)
+        g.n_tiles += ((c.width + both->TW - 1) / both->TW) * ((c.height + both->TH - 1) / both->TH);
+      p->all.src.insert(p->all.src.end(), g.src.begin(), g.src.end());
+      p->all.n_images += g.n_images;
+    } else if (vs[cls]) {
       st = seg_build(p, g, vs[cls], s);
-    } else {
-      seg_free(g);
-      g.n_tiles = 0;
     }
   }
-  if (st == SATGB_OK) st = plan_merge(p, s);
+  if (st == SATGB_OK && both) st = seg_build(p, p->all, both, s);
   if (st == SATGB_OK) st = plan_ws(p, s);
   return st;
 }
@@ -1522,8 +1517,9 @@ satgb_status satgb_batch_plan_create(satgb_batch_plan** plan, satgb_dtype in_t, 
       cfgs[cls] = it != g_batch_tune.end() ? it->second : batch_default_config(p, cls);
     }
     vs[cls] = seg_variant(p, cls, cfgs[cls]);
+    if (!vs[cls]) st = fail(SATGB_ERR_UNSUPPORTED_TYPES, "no kernel for this batch");
   }
-  st = plan_layout(p, vs, s);
+  if (st == SATGB_OK) st = plan_layout(p, vs, s);
   if (st == SATGB_OK && p->n_tiles > 0) st = plan_capture(p);
   if (st != SATGB_OK) {
     plan_free(p);

@@ -1099,3 +1099,49 @@ def test_both_kernels_of_configuration_5(cuda, t):
         sat_gb300.stream_check()
     finally:
         sat_gb300.set_config(-1)
+
+
+def test_plan_of_one_launch_keeps_one_table(cuda):
+    """A plan whose classes share a launch holds the tile order (16 bytes a tile) of that launch and
+    none of the classes' own: 64 columns of 2^20 pixels, half a million tiles, and a small image."""
+    L = _lib.load()
+    n, h = 64, 1 << 20
+    ins = torch.ones((n, h, 1), dtype=torch.uint8, device=cuda)
+    outs = torch.zeros((n, h, 1), dtype=torch.int32, device=cuda)
+    small, small_out = torch.ones((50, 60), dtype=torch.uint8, device=cuda), torch.zeros((50, 60), dtype=torch.int32, device=cuda)
+    pool = torch.empty(3 << 30, dtype=torch.uint8, device=cuda)  # the plans' workspaces
+    at = [0]
+
+    def alloc(size, ctx):
+        p = pool.data_ptr() + at[0]
+        at[0] += (size + 4095) // 4096 * 4096
+        return p if at[0] <= pool.numel() else 0
+
+    hooks = _lib._ALLOC_FN(alloc), _lib._FREE_FN(lambda p, ctx: None)
+
+    def plan(k):
+        return sat_gb300.BatchPlan([ins[i] for i in range(k)] + [small],
+                                   [outs[i].view(torch.uint32) for i in range(k)] + [small_out.view(torch.uint32)])
+
+    sat_gb300.release()
+    assert L.satgb_set_allocator(*hooks, None) == 0
+    try:
+        first = plan(1)  # the kernels and the graph's own memory
+        first.exec()
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        p = plan(n)
+        held = free - torch.cuda.mem_get_info()[0]
+        c = p.classes()
+        assert c[0]["config"] == c[1]["config"] and c[0]["tiles"] == n * (h // 128) and c[1]["tiles"] == 1
+        assert held < 1.5 * 16 * c[0]["tiles"], held
+        p.exec()
+        p.check()
+        want = torch.arange(1, h + 1, dtype=torch.int32, device=cuda)
+        assert all(torch.equal(outs[i, :, 0], want) for i in range(n))
+        assert int(small_out[-1, -1]) == 3000
+        p.close()
+        first.close()
+    finally:
+        torch.cuda.synchronize()
+        assert L.satgb_set_allocator(_lib._ALLOC_FN(), _lib._FREE_FN(), None) == 0
