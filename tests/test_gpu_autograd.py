@@ -500,3 +500,19 @@ def test_box_layer_both_ways(cuda, shape, radii, scratch):
             dtol += window_error(min(r, max(H, W) - 1)) + 8 * EPS32 * 4 * float(w[n, k].abs().sum()) / area
         err = float((dx[n].double() - dx64).abs().max())
         assert err <= dtol, (n, err, dtol)
+
+
+def test_box_layer_error_is_that_of_windows(cuda):
+    """Rounding errors of the one-launch kernels stay those of window sums: over N(0, 1) planes of 1024^2 a column's running sum
+    (|V| about sqrt(2r + 1)) takes 256 roundings, which add as a random walk, and a prefix of 256 of them a few more, 3e-7
+    of a mean's unit in all (standard deviation, radius 3); bound: 17 of those, for the three radii's gradient sqrt(3)
+    times as many.  Through the SAT, whose values reach thousands, the largest error is several times the bound."""
+    g = torch.Generator(device="cpu").manual_seed(71)
+    x = torch.randn((3, 1024, 1024), generator=g).to(cuda)
+    w = torch.randn((3, 3, 1024, 1024), generator=g).to(cuda)
+    radii = (3, 7, 15)
+    x64 = x.double().requires_grad_(True)
+    m64 = box_means64(x64, radii)
+    (dx64,) = torch.autograd.grad(m64, x64, w.double())
+    assert float((api.box_means(x, radii).double() - m64).abs().max()) <= 5e-6
+    assert float((api.box_means_grad_x(w, radii).double() - dx64).abs().max()) <= 9e-6

@@ -1145,3 +1145,31 @@ def test_plan_of_one_launch_keeps_one_table(cuda):
     finally:
         torch.cuda.synchronize()
         assert L.satgb_set_allocator(_lib._ALLOC_FN(), _lib._FREE_FN(), None) == 0
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan")])
+def test_infinities_leave_finite_sums_exact(cuda, value):
+    """An infinity's sign and a NaN arrive in every sum that contains them, and every other sum is what it is without them, to the
+    bit (sums of ones below 2^24): both kernels of configuration 5, aligned, packed and offset rows, both directions, and
+    column scans by strips and by tiles, with and without a partial last strip."""
+    def same(got, want):
+        finite = want.isfinite()
+        return (torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isposinf(), want.isposinf())
+                and torch.equal(got.isneginf(), want.isneginf()) and torch.equal(got[finite], want[finite]))
+
+    try:
+        for h, w, off in [(500, 512, 0), (601, 389, 0), (300, 250, 1), (3000, 40, 0), (1030, 1001, 0), (8200, 100, 0)]:
+            x = torch.ones((h, w + 4 * off), device=cuda)[:, off:off + w]
+            for r, c in [(h // 2, w // 3), (0, 0), (h - 1, w - 1)]:
+                y = x.clone() if not off else torch.ones((h, w + 4), device=cuda)[:, 1:1 + w]
+                y[r, c] = value
+                assert same(sat_gb300.scan_cols(y, torch.float32), y.double().cumsum(0).float()), (h, w)
+                sats = y.double().cumsum(0).cumsum(1).float()
+                sat_gb300.set_config(5)
+                assert same(sat_gb300.sat(y, torch.float32), sats), (h, w)
+                flipped = torch.ones((h, w + 4 * off), device=cuda)[:, off:off + w]
+                flipped.copy_(y.flip((0, 1)))
+                assert same(sat_gb300.sat(flipped, torch.float32, reverse=True).flip((0, 1)), sats), (h, w)
+                sat_gb300.set_config(-1)
+    finally:
+        sat_gb300.set_config(-1)
