@@ -212,10 +212,11 @@ int satgb_box_filter_fwd_x_scratch(const satgb_box_desc* desc);
 satgb_status satgb_box_filter_bwd(const satgb_box_desc* desc, satgb_stream stream);
 /* The gradient of the box means with respect to the image the SAT was taken
  * of, in one call and without scratch memory: one launch of window sums of the
- * means' gradients, or, for radii too large for that kernel's shared memory,
+ * means' gradients, or, where that is faster (large radii, narrow planes),
  * dL/dSAT gathered into d_dx and reverse-summed in place (two tile launches
- * and the edge launch of satgb_box_filter_bwd).  desc->d_sat is not used; d_dx (n_planes planes of width x height, pitch and plane stride in
- * elements) is written and may not overlap the gradients of the means. */
+ * and the edge launch of satgb_box_filter_bwd).  desc->d_sat is not used; d_dx
+ * (n_planes planes of width x height, pitch and plane stride in elements) is
+ * written and may not overlap the gradients of the means. */
 satgb_status satgb_box_filter_bwd_x(const satgb_box_desc* desc, void* d_dx, int64_t dx_pitch,
                                     int64_t dx_plane_stride, satgb_stream stream);
 
@@ -280,11 +281,15 @@ satgb_status satgb_batch_plan_info(const satgb_batch_plan* plan, int64_t* n_tile
 satgb_status satgb_batch_plan_classes(const satgb_batch_plan* plan, int64_t* n_images, int64_t* n_tiles,
                                       int* configs);
 /* Batch autotuner: times every tile configuration of each size class on the
- * plan's own images (launches whose results overwrite the outputs), keeps the
+ * plan's own images (launches whose results overwrite the outputs), each laid
+ * out as a plan that takes it (with the copies of inputs that it needs), and, where the
+ * classes prefer different ones, either one for both in one launch; keeps the
  * fastest, records it in the tuning cache under the batch's signature (dtype
- * pair, mode, direction, class, pixel and image counts, TMA alignment of the
+ * pair, mode, direction, class, pixel and image counts, alignment of the
  * rows, SM count; persisted in SATGB_TUNE_CACHE when set) and captures the
- * plan's graph again.  configs may be NULL or receive the 2 chosen indices. */
+ * plan's graph again.  After an error the plan is what it was, or, where that
+ * failed too, its exec and launch return an error.  configs may be NULL or
+ * receive the 2 chosen indices. */
 satgb_status satgb_batch_plan_autotune(satgb_batch_plan* plan, satgb_stream stream, int* configs);
 /* Synchronises `stream` and reports (and clears) a device-side error of the
  * plan's launches, like satgb_stream_check does for single-image calls. */

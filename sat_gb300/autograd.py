@@ -7,10 +7,11 @@ so dL/dI(i,j) = sum_{y >= i, x >= j} dL/dS(y,x): the suffix (reverse) SAT of
 the incoming gradient, one launch of the same kernel with direction=reverse.
 
 Box filter.  box_filter_means(x, radii) returns the clipped box means of every
-radius, read by four corners from the SAT of x (one SAT launch plus one box
-launch forward).  Backward: the adjoint gather into the gradient tensor,
-then the reverse SAT of that tensor in place (the plain mode in one call of
-the library, the compensated mode with the compensated reverse SAT).
+radius.  The plain mode takes them, and their gradient, each in one launch of
+window sums without a SAT, or through the SAT where that is faster (one call of
+the library either way).  The compensated mode reads the four corners of the
+compensated SAT of x; its backward is the adjoint gather and the compensated reverse
+SAT in place.
 """
 from __future__ import annotations
 
@@ -51,9 +52,9 @@ def sat(x: torch.Tensor, mode: str = "plain") -> torch.Tensor:
 
 
 class BoxMeansFunction(torch.autograd.Function):
-    """(..., H, W) -> (..., R, H, W): clipped box means of radius radii[k],
-    computed from the SAT of x.  Backward: the four-corner adjoint (a gather)
-    gives dL/dSAT, whose reverse SAT is dL/dx."""
+    """(..., H, W) -> (..., R, H, W): clipped box means of radius radii[k] of
+    x, from its window sums or its SAT; backward: dL/dx, from the window sums of
+    the means' gradients or as the reverse SAT of dL/dSAT."""
 
     @staticmethod
     def forward(ctx, x: torch.Tensor, radii: tuple, mode: str = "plain"):
@@ -69,7 +70,7 @@ class BoxMeansFunction(torch.autograd.Function):
     def backward(ctx, g: torch.Tensor):
         g = _as_f32_cuda(g)
         if ctx.mode == "plain":
-            # adjoint gather and in-place reverse SAT in one library call
+            # window sums, or adjoint gather and in-place reverse SAT, in one library call
             return api.box_means_grad_x(g, ctx.radii), None, None
         gs = api.box_means_adjoint(g, ctx.radii)
         # the reverse SAT may overwrite its input in place: gs is ours alone

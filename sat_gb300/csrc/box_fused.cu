@@ -206,8 +206,8 @@ __device__ __forceinline__ int warp_id() { return __shfl_sync(0xffffffffu, (int)
 // once a batch of kDMeans rows, whose scans go side by side kPMeans at a time; copies
 // run sh.ahead batches ahead.  64 x 3 x 1024^2, radii 3, 7, 15, us by (kDMeans, kPMeans):
 // (2, 2) 765, (4, 2) 780, (2, 1) 790, (4, 1) 792, (8, 1) 846; through the SAT 1210.
-// The shared-memory pipe bounds it (68 % of its wavefronts busy: per output and radius
-// two ring reads, one prefix written and two read), then its own latency at 15 warps an SM.
+// The shared-memory pipe bounds it (67 % of its wavefronts busy: per output and radius
+// two ring reads, one prefix written and two read), then its own latency at 13 warps an SM (issue slots 50 % busy).
 constexpr int kDMeans = 2, kPMeans = 2;
 
 // The outputs of D rows (of the first `rows` of them): G groups of 32 columns and, in lanes below `rest`,
@@ -327,8 +327,8 @@ __global__ void __launch_bounds__(NR * 32) box_means_kernel(const __grid_constan
 // The gradient: every radius has its own gradient plane and ring; the radii's
 // window sums meet in shared memory, a batch at a time, and the warps share the
 // outputs, one group of 32 columns of a row after the other.  64 x 3 x 1024^2, radii
-// 3, 7, 15: 990 us (dL/dSAT and its reverse SAT: 1320), bound by latency at 9 warps an
-// SM (the rings' 53 rows of 1 KB leave room for three blocks).
+// 3, 7, 15: 1020 us (dL/dSAT and its reverse SAT: 1320; 1000 with the sums from the first row and column on), bound by
+// latency at 8.4 warps an SM (the rings leave room for three blocks; issue slots 41 % busy).
 constexpr int kDGrad = 2;
 
 template <int NR, bool VEC>

@@ -1,5 +1,5 @@
 // sat_kernel_wd.cuh -- the warp-specialized tile loop for 1-byte and 4-byte inputs with 4-byte sums
-// (configuration 5 for those pairs).
+// (configuration 5 for those pairs; 4-byte inputs also have 128-row tiles there, config5_kernel in satgb_api.cu).
 //
 // A tile's data flow is that of sat_kernel_ws.cuh with direct stores.  What bounds that kernel for 8-bit
 // pixels is not memory (u8 -> u32 8192^2: 99.7 us, floor 49.5): with its stores left out it is as

@@ -14,7 +14,8 @@
 // warps of 16 rows and each warp adding up the ones before it a block took 2 us, and f32 errors doubled; an f32
 // column's sum over the blocks is a two-sum pair (mean relative error at 8192 rows 7.9e-8 -> 4.6e-8).
 // us in a graph, look-back over tiles and strips: f32 256 x 256 8.0 and 3.1, 1024^2 10.1 and 6.2, 4096 x 2048 18.1 and
-// 11.1, 4096^2 33.6 and 28.7, packed 3001 x 3003 33.4 and 17.6, 8191^2 220 and 143; f64 4096^2 177 and 116.
+// 11.1, 4096^2 33.6 and 28.7, packed 3001 x 3003 33.4 and 17.6, 8191^2 221 and 129; f64 4096^2 177 and 116.  On
+// buffers used in turn 4096^2 is 32.0: of the same two, 134 MB, L2 keeps a part.
 #include <cuda_runtime.h>
 
 #include <algorithm>
