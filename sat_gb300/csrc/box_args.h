@@ -34,6 +34,6 @@ satgb_status box_check_desc(const satgb_box_desc* d, BoxArgs& a);
 // memory or, unless `only_way`, going through the SAT is faster: the
 // caller then does that.  launch false: only *done.
 satgb_status box_means_fused(const BoxArgs& a, cudaStream_t s, bool only_way, bool launch, bool* done);
-satgb_status box_grad_fused(const BoxArgs& a, cudaStream_t s, bool* done);
+satgb_status box_grad_fused(const BoxArgs& a, cudaStream_t s, bool only_way, bool* done);
 
 }  // namespace satgb

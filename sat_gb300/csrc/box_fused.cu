@@ -597,7 +597,7 @@ satgb_status box_means_fused(const BoxArgs& a, cudaStream_t s, bool only_way, bo
   return SATGB_OK;
 }
 
-satgb_status box_grad_fused(const BoxArgs& a, cudaStream_t s, bool* done) {
+satgb_status box_grad_fused(const BoxArgs& a, cudaStream_t s, bool only_way, bool* done) {
   *done = false;
   Shape sh;
   int64_t smem = grad_smem(a, sh.ahead = 1);
@@ -605,7 +605,7 @@ satgb_status box_grad_fused(const BoxArgs& a, cudaStream_t s, bool* done) {
   const int blocks = resident(smem);
   sh.tx = columns(a);
   sh.sy = strip_rows(a, sh.tx, blocks);
-  *done = pays(a, sh, blocks, true);
+  *done = only_way || pays(a, sh, blocks, true);
   if (!*done) return SATGB_OK;
   if (resident(grad_smem(a, 2)) == blocks && grad_smem(a, 2) <= kMaxSmem) smem = grad_smem(a, sh.ahead = 2);
   bool vec = true;

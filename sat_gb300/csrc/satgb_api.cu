@@ -664,6 +664,33 @@ satgb_status scan_cols_strips(int in_t, int out_t, const void* d_in, int64_t in_
 namespace {
 constexpr int kModeCols = 3;
 
+// Whether a launch of `v` on `s` has its look-back workspace or may allocate it: it may not while the stream is captured.  A call
+// that has a way without a workspace takes that then, whichever is faster.  Called with g_mu held.
+bool ws_at_hand(const Variant* v, long long width, long long height, long long planes, int dev, cudaStream_t s) {
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &capture) != cudaSuccess) {
+    cudaGetLastError();
+    return true;
+  }
+  if (capture == cudaStreamCaptureStatusNone || !v) return true;
+  auto it = g_ws.find(std::make_pair(dev, (void*)s));
+  const long long tiles = ((width + v->TW - 1) / v->TW) * ((height + v->TH - 1) / v->TH) * planes;
+  return it != g_ws.end() && it->second.bytes >= layout_for(tiles, v).total;
+}
+
+// The same of a plain f32 SAT, for the box calls.
+bool sat_ws_at_hand(int dir, long long width, long long height, long long planes, cudaStream_t s) {
+  std::lock_guard<std::mutex> lk(g_mu);
+  int dev = 0;
+  if (get_device(&dev) != SATGB_OK) return true;
+  const int cfg = choose_config_locked(SATGB_F32, SATGB_F32, SATGB_MODE_PLAIN, dir, width, height, dev, planes,
+                                       planes == 1 && width % 4 != 0);
+  const Variant* v = find_variant(SATGB_F32, SATGB_F32, SATGB_MODE_PLAIN, dir, cfg);
+  return ws_at_hand(v, width, height, planes, dev, s) &&
+         (cfg != 5 || ws_at_hand(find_variant(SATGB_F32, SATGB_F32, SATGB_MODE_PLAIN, dir, kConfig5Wide), width, height, planes,
+                                 dev, s));
+}
+
 satgb_status sat_single(int in_t, int out_t, int mode, int dir, const void* d_in, long long in_pitch,
                         void* d_out, long long out_pitch, long long width, long long height,
                         cudaStream_t s, int force_cfg, long long planes = 1, long long in_plane = 0,
@@ -709,7 +736,8 @@ satgb_status sat_single(int in_t, int out_t, int mode, int dir, const void* d_in
   if (st != SATGB_OK) return st;
   // ... nor has the column-only scan of wide images (scan_cols.cu)
   if (mode == kModeCols && dir == SATGB_FORWARD && planes == 1 &&
-      scan_cols_by_strips(d_in, in_pitch, in_sz, d_out, out_pitch, out_sz, width, height, sms_of(dev)))
+      (scan_cols_by_strips(d_in, in_pitch, in_sz, d_out, out_pitch, out_sz, width, height, sms_of(dev)) ||
+       !ws_at_hand(find_variant(in_t, out_t, mode, dir, 1), width, height, 1, dev, s)))
     return scan_cols_strips(in_t, out_t, d_in, in_pitch, d_out, out_pitch, width, height, s);
   const bool off16 = planes == 1 && in_pitch == width && (uintptr_t)d_in % 16 == 0 && ((size_t)in_pitch * in_sz) % 16 != 0;
   int cfg = force_cfg >= 0 ? force_cfg
@@ -1083,6 +1111,8 @@ satgb_status satgb_box_filter_fwd_x(const satgb_box_desc* desc, const void* d_x,
   }
   bool done = false;
   st = satgb::box_means_fused(a, (cudaStream_t)stream, !desc->d_sat, true, &done);
+  if (st == SATGB_OK && !done && desc->d_sat && !sat_ws_at_hand(SATGB_FORWARD, w, h, planes, (cudaStream_t)stream))
+    st = satgb::box_means_fused(a, (cudaStream_t)stream, true, true, &done);
   if (st != SATGB_OK || done) return st;
   if (!desc->d_sat)
     return fail(SATGB_ERR_NOT_FOUND, "box means: radii above 64 need a scratch SAT (descriptor's d_sat)");
@@ -1126,7 +1156,9 @@ satgb_status satgb_box_filter_bwd_x(const satgb_box_desc* desc, void* d_dx, int6
   satgb_status st = satgb::box_check_desc(&d, a);
   if (st != SATGB_OK) return st;
   bool done = false;
-  st = satgb::box_grad_fused(a, (cudaStream_t)stream, &done);
+  st = satgb::box_grad_fused(a, (cudaStream_t)stream, false, &done);
+  if (st == SATGB_OK && !done && !sat_ws_at_hand(SATGB_REVERSE, w, h, planes, (cudaStream_t)stream))
+    st = satgb::box_grad_fused(a, (cudaStream_t)stream, true, &done);
   if (st != SATGB_OK || done) return st;
   // dL/dSAT into the output, then its reverse SAT in place
   st = satgb_box_filter_bwd(&d, stream);
