@@ -326,8 +326,9 @@ __global__ void __launch_bounds__(NR * 32) box_means_kernel(const __grid_constan
 // ---------------------------------------------------------------------------
 // The gradient: every radius has its own gradient plane and ring; the radii's
 // window sums meet in shared memory, a batch at a time, and the warps share the
-// outputs, one group of 32 columns of a row after the other.  64 x 3 x 1024^2, radii
-// 3, 7, 15: 1020 us (dL/dSAT and its reverse SAT: 1320; 1000 with the sums from the first row and column on), bound by
+// outputs, one group of 32 columns of a row after the other.  The launch hands the planes over upside down
+// (flipped), so rows here go from the last one up.  64 x 3 x 1024^2, radii
+// 3, 7, 15: 1004 us (dL/dSAT and its reverse SAT: 1320; with rows counted down here instead 1020), bound by
 // latency at 8.4 warps an SM (the rings leave room for three blocks; issue slots 41 % busy).
 constexpr int kDGrad = 2;
 
@@ -339,7 +340,9 @@ __global__ void __launch_bounds__(NR * 32) box_grad_kernel(const __grid_constant
   const int W = (int)a.w, H = (int)a.h, R = a.rmax;
   const int lane = threadIdx.x & 31, k = warp_id();
   const int X0 = blockIdx.x * sh.tx, y0 = blockIdx.y * sh.sy, y1 = min(H, y0 + sh.sy);
-  const int xs = (X0 - R - 1) & ~3;
+  // The sums run from the last column back: the block's last columns are the last ones that its outputs need, so that
+  // no others enter (tx + 2 R + 1 <= 253, or 255 where R + 1 is a multiple of 4: the first needed one is there too).
+  const int xs = (X0 + sh.tx + R - kW + 3) & ~3;
   const int r = a.r[k];
   const float inv = a.inv_full[k];
   float* ring = smem + D * NR * kW;
@@ -348,11 +351,11 @@ __global__ void __launch_bounds__(NR * 32) box_grad_kernel(const __grid_constant
     if (i < k) ring += (2 * a.r[i] + 1 + (1 + sh.ahead) * D) * kW;
   const int wrap = (2 * r + 1 + (1 + sh.ahead) * D) * kW;
   const float* src = a.box[k] + (int64_t)blockIdx.z * a.box_plane;
-  int jn = y1 + r, jslot = 0;
+  int jn = y0 - r - 1, jslot = 0;
   auto copy = [&](int n) {
-    if (jn >= y0 - r) {
-      for (int i = 0; i < n; ++i, --jn) {
-        copy_row<VEC, 32>(ring + jslot, src + (int64_t)jn * a.box_pitch, src, xs, W, jn >= max(0, y0 - r) && jn < H, lane);
+    if (jn < y1 + r) {
+      for (int i = 0; i < n; ++i, ++jn) {
+        copy_row<VEC, 32>(ring + jslot, src + (int64_t)jn * a.box_pitch, src, xs, W, jn >= 0 && jn < min(H, y1 + r), lane);
         jslot += kW;
         if (jslot == wrap) jslot = 0;
       }
@@ -387,9 +390,9 @@ __global__ void __launch_bounds__(NR * 32) box_grad_kernel(const __grid_constant
     const int i = (t0 + t) / ng, c = (t0 + t) - i * ng;
     pi[t] = t < nt && c * 32 + lane < n ? i : H;
     ps[t] = t < nt ? i * (NR * kW) + c * 32 : 0;
-    po[t] = c * 32 - i * a.sat_pitch;
+    po[t] = c * 32 + i * a.sat_pitch;
   }
-  float* out = a.sat + (int64_t)blockIdx.z * a.sat_plane + (int64_t)(y1 - 1) * a.sat_pitch + X0 + lane;
+  float* out = a.sat + (int64_t)blockIdx.z * a.sat_plane + (int64_t)y0 * a.sat_pitch + X0 + lane;
 
   F2 V[4];
 #pragma unroll
@@ -397,30 +400,30 @@ __global__ void __launch_bounds__(NR * 32) box_grad_kernel(const __grid_constant
   int sout = 0, sin = (2 * r + 1) * kW;
   copies_wait_ahead(sh.ahead);
   __syncthreads();
-  for (int i = 0; i <= 2 * r; ++i) { // the window of row y1
+  for (int i = 0; i <= 2 * r; ++i) { // the window of row y0 - 1
     F2 e[4];
     ring_read(e, mine + i * kW, d);
-    const float f = clipped_inv(min(max(y1 + r - i, 0), H - 1), r, H, inv);
+    const float f = clipped_inv(min(max(y0 - r - 1 + i, 0), H - 1), r, H, inv);
 #pragma unroll
     for (int q = 0; q < 4; ++q) V[q] = fma2(f2(f, f), e[q], V[q]);
   }
 #pragma unroll 1
-  for (int yb = y1 - 1; yb >= y0; yb -= D) {
+  for (int yb = y0; yb < y1; yb += D) {
     copies_wait_ahead(sh.ahead - 1);
     __syncthreads(); // the last batch's prefix rows have been read; this batch's rows have arrived
     copy(D);
-    const bool yinner = yb - (D - 1) - 2 * r >= 0 && yb + 2 * r + 1 <= H - 1;
+    const bool yinner = yb - 2 * r - 1 >= 0 && yb + D - 1 + 2 * r <= H - 1;
     F2 u[D][4];
 #pragma unroll
     for (int i = 0; i < D; ++i) {
-      const int y = yb - i;
+      const int y = yb + i;
       F2 e[4], l[4];
       ring_read(e, mine + sin, d);
       ring_read(l, mine + sout, d);
       float fe = inv, fl = inv;
       if (!yinner) {
-        fe = clipped_inv(min(max(y - r, 0), H - 1), r, H, inv);
-        fl = clipped_inv(min(max(y + r + 1, 0), H - 1), r, H, inv);
+        fe = clipped_inv(min(max(y + r, 0), H - 1), r, H, inv);
+        fl = clipped_inv(min(max(y - r - 1, 0), H - 1), r, H, inv);
       }
 #pragma unroll
       for (int q = 0; q < 4; ++q) V[q] = fma2(f2(-fl, -fl), l[q], fma2(f2(fe, fe), e[q], V[q]));
@@ -439,9 +442,9 @@ __global__ void __launch_bounds__(NR * 32) box_grad_kernel(const __grid_constant
       float s = ld[0][ps[t]] - rd[0][ps[t]];
 #pragma unroll
       for (int q = 1; q < NR; ++q) s += ld[q][ps[t]] - rd[q][ps[t]];
-      if (yb - pi[t] >= y0) __stcs(out + po[t], s);
+      if (yb + pi[t] < y1) __stcs(out + po[t], s);
     }
-    out -= D * a.sat_pitch;
+    out += D * a.sat_pitch;
   }
 }
 
@@ -573,6 +576,16 @@ bool pays(const BoxArgs& a, const Shape& sh, int blocks, bool grad) {
   return R <= 31 && (a.nr > 1 || off16 || R <= 27 || across * kW * 100 <= w * 155);
 }
 
+// The same planes from their last row up: windows are symmetric, and so are their clipped lengths.
+BoxArgs flipped(const BoxArgs& a) {
+  BoxArgs f = a;
+  f.sat += (a.h - 1) * a.sat_pitch;
+  f.sat_pitch = -a.sat_pitch;
+  for (int k = 0; k < a.nr; ++k) f.box[k] += (a.h - 1) * a.box_pitch;
+  f.box_pitch = -a.box_pitch;
+  return f;
+}
+
 }  // namespace
 
 namespace satgb {
@@ -610,7 +623,8 @@ satgb_status box_grad_fused(const BoxArgs& a, cudaStream_t s, bool only_way, boo
   if (resident(grad_smem(a, 2)) == blocks && grad_smem(a, 2) <= kMaxSmem) smem = grad_smem(a, sh.ahead = 2);
   bool vec = true;
   for (int k = 0; k < a.nr; ++k) vec = vec && rows_vec(a.box[k], a.w, a.box_pitch, a.box_plane, a.planes);
-  const cudaError_t e = vec ? launch_grad<true>(a, sh, (int)smem, s) : launch_grad<false>(a, sh, (int)smem, s);
+  const BoxArgs f = flipped(a);
+  const cudaError_t e = vec ? launch_grad<true>(f, sh, (int)smem, s) : launch_grad<false>(f, sh, (int)smem, s);
   if (e != cudaSuccess) return api_cuda_fail(e, "box_grad_kernel launch");
   api_count_launch();
   return SATGB_OK;
