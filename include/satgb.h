@@ -199,7 +199,7 @@ satgb_status satgb_box_filter_fwd(const satgb_box_desc* desc, satgb_stream strea
  * writes no SAT.  Without a scratch SAT (desc->d_sat NULL) every set of radii up
  * to 64 is taken so, and larger ones (as clamped to max(width, height) - 1)
  * return SATGB_ERR_NOT_FOUND.  With one (d_sat with its pitch and plane stride) the call
- * takes any radii, and goes through the SAT where that is the faster way.
+ * takes any radii, and goes through the SAT for large ones, which is faster.
  * The means may not overlap the image. */
 satgb_status satgb_box_filter_fwd_x(const satgb_box_desc* desc, const void* d_x, int64_t x_pitch,
                                     int64_t x_plane_stride, satgb_stream stream);
@@ -212,7 +212,7 @@ int satgb_box_filter_fwd_x_scratch(const satgb_box_desc* desc);
 satgb_status satgb_box_filter_bwd(const satgb_box_desc* desc, satgb_stream stream);
 /* The gradient of the box means with respect to the image the SAT was taken
  * of, in one call and without scratch memory: one launch of window sums of the
- * means' gradients, or, where that is faster (large radii, narrow planes),
+ * means' gradients, or, for large radii,
  * dL/dSAT gathered into d_dx and reverse-summed in place (two tile launches
  * and the edge launch of satgb_box_filter_bwd).  desc->d_sat is not used; d_dx
  * (n_planes planes of width x height, pitch and plane stride in elements) is

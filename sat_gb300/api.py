@@ -282,8 +282,8 @@ def box_means(x: torch.Tensor, radii: Sequence[int], out=None, stream=None) -> t
     dx, pitch, plane = d.d_sat, d.sat_pitch, d.sat_plane_stride
     d.d_sat = None
     fwd, handle, scratch = _lib.load().satgb_box_filter_fwd_x, _call_stream(stream), None
-    # (up to radius 15 the library never takes it)
-    if max(d.radius) > 15 and _lib.load().satgb_box_filter_fwd_x_scratch(ctypes.byref(d)):
+    # (up to radius 33 the library never takes it)
+    if max(d.radius) > 33 and _lib.load().satgb_box_filter_fwd_x_scratch(ctypes.byref(d)):
         # from the pool of the stream that uses it: the block goes back, and to its next owner, in that
         # stream's order, whatever stream is current
         scratch = torch.cuda.caching_allocator_alloc(4 * x.numel(), x.device, handle)

@@ -31,7 +31,7 @@ satgb_status box_check_desc(const satgb_box_desc* d, BoxArgs& a);
 // their gradient with respect to the image straight from the means' gradients
 // (`a.sat` is the gradient written), each in one launch.  *done is false, and
 // nothing was launched, when the radii are too large for the kernels' shared
-// memory or, unless `only_way`, going through the SAT is faster: the
+// memory or, unless `only_way`, for going in one launch to be the faster way: the
 // caller then does that.  launch false: only *done.
 satgb_status box_means_fused(const BoxArgs& a, cudaStream_t s, bool only_way, bool launch, bool* done);
 satgb_status box_grad_fused(const BoxArgs& a, cudaStream_t s, bool only_way, bool* done);

@@ -544,36 +544,18 @@ cudaError_t launch_grad(const BoxArgs& a, const Shape& sh, int smem, cudaStream_
   }
 }
 
-// Whether one launch is faster than going through the SAT, for a.w x a.h planes whose blocks are `sh` and stand
-// `blocks` to an SM.  Measured with both ways forced, 16 to 2048 columns, radii 7 to 60 alone and with smaller ones, totals of
-// 1, 12 and 150 million pixels; ratios below are this way's time over the SAT's.
-// - Few resident blocks leave too few warps to hide the scans' latency, and a block computes 256 columns for `most`
-//   (columns()) at best: 224 up to radius 15, 192 to 31, 160 to 47.  Up to radius 23 this way wins wherever a plane is not much
-//   narrower than a block's reach (0.4 to 0.95); narrow planes lose (16 columns: radius 23 1.1 to 1.7; 64: radius 31 1.0 to 1.25),
-//   rows off 16-byte boundaries later, as the SAT's tiles are slower there.
-// - A call that does not fill the SMs once is bound by its launches, of which this way has one (0.3 to 0.8).
-// - Planes that fill half of the SAT's 128 x 128 tiles or less (160 columns) are slower there (0.7 to 0.9 at any radius).
-// - Beyond radius 23 the means alone win to radius 27, and to 31 where the blocks' columns are used (900 columns 0.86, 1024
-//   0.99; 256 1.25), of several radii to 31 (0.8 to 1.05; radius 34 1.15 to 1.57).  The gradient of one radius
-//   wins to 29 (31: 0.9 to 1.17), of two to 31 (0.9 to 1.13), of four to 31 (0.7 to 1.07), and to 45 below 1000 columns
-//   (0.7 to 0.99).
-bool pays(const BoxArgs& a, const Shape& sh, int blocks, bool grad) {
-  const int64_t w = a.w, h = a.h;
-  const int R = a.rmax;
-  if (!(grad ? blocks >= 3 || (blocks == 2 && a.nr >= 2) || a.nr == 4 : blocks >= 3 || (blocks == 2 && a.nr >= 3)))
-    return false;
-  const bool off16 = w % 4 != 0;
-  if (R > 15 && (off16 ? R * 100 > 75 * w || (R > 23 && R * 100 > 47 * w) : R * 100 > 47 * w)) return false;
-  if (R <= 23) return true;
-  const int64_t across = (w + sh.tx - 1) / sh.tx;
-  if (across * a.planes * ((h + sh.sy - 1) / sh.sy) <= (int64_t)device_sms() * blocks) return true;
-  if (((w + 127) & ~127LL) * ((h + 127) & ~127LL) >= 2 * w * h) return true;
-  if (grad) {
-    if (a.nr == 4) return R <= 31 || (R <= 45 && w < 1000) || w < 450;
-    return R <= 29 || (R <= 31 && (off16 || a.nr == 2)) || (a.nr == 2 && across == 1);
-  }
-  if (a.nr == 4 && (off16 || (across == 1 && w >= 100))) return true;
-  return R <= 31 && (a.nr > 1 || off16 || R <= 27 || across * kW * 100 <= w * 155);
+// Whether a call whose blocks stand `blocks` to an SM goes in one launch.  Few blocks leave too few warps to hide the scans'
+// latency.  Measured on 8 x 3 x 700 x 900 (us, these kernels / through the SAT), by blocks an SM:
+//   means     1: radius 64 366 / 90        2: radii 5, 11, 21, 31 158 / 158 (3 blocks: 109), 45, 46, 47 179 / 135
+//             3: radius 31 67 / 81, radii 21, 31 87 / 107, radius 33 86 / 82
+//   gradient  1: radii 21, 31 240 / 168, radii 5, 11, 21, 31 254 / 274
+//             2: radii 3, 31 144 / 152     3: radius 31 95 / 108
+// Over 900 sizes (16 to 2048 columns, radii 7 to 60, 1 to 150 million pixels) the SAT is the faster way within these lines too for
+// planes narrower than twice the radius (16 columns, radius 23: 1.1 to 1.7 times as fast), for radii above 31, where a block
+// computes 256 columns for 160 (1.1 to 1.6 in calls that fill the SMs), and for one radius of 28 to 31 below 512 columns (1.0 to 1.25).
+// Those calls stay here all the same: their errors are those of a window (5e-7 of the means' norm), the SAT's 20 times as large.
+bool one_launch(int nr, int blocks, bool grad) {
+  return grad ? blocks >= 3 || (blocks == 2 && nr >= 2) || nr == 4 : blocks >= 3 || (blocks == 2 && nr >= 3);
 }
 
 // The same planes from their last row up: windows are symmetric, and so are their clipped lengths.
@@ -599,7 +581,7 @@ satgb_status box_means_fused(const BoxArgs& a, cudaStream_t s, bool only_way, bo
   const int blocks = resident(smem);
   sh.tx = columns(a);
   sh.sy = strip_rows(a, sh.tx, blocks);
-  *done = only_way || pays(a, sh, blocks, false);
+  *done = only_way || one_launch(a.nr, blocks, false);
   if (!*done || !launch) return SATGB_OK;
   if (resident(means_smem(a, 2)) == blocks) smem = means_smem(a, sh.ahead = 2);
   const cudaError_t e = rows_vec(a.sat, a.w, a.sat_pitch, a.sat_plane, a.planes)
@@ -618,7 +600,7 @@ satgb_status box_grad_fused(const BoxArgs& a, cudaStream_t s, bool only_way, boo
   const int blocks = resident(smem);
   sh.tx = columns(a);
   sh.sy = strip_rows(a, sh.tx, blocks);
-  *done = only_way || pays(a, sh, blocks, true);
+  *done = only_way || one_launch(a.nr, blocks, true);
   if (!*done) return SATGB_OK;
   if (resident(grad_smem(a, 2)) == blocks && grad_smem(a, 2) <= kMaxSmem) smem = grad_smem(a, sh.ahead = 2);
   bool vec = true;

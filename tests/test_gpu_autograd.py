@@ -465,12 +465,11 @@ def test_box_layer_infinities_spoil_no_more_than_the_sat_path(cuda, shape, radii
 
 
 @pytest.mark.parametrize("shape,radii,scratch", [
-    ((4, 64, 16), (15,), 0), ((4, 64, 16), (16,), 1), ((4, 64, 33), (23,), 0), ((4, 64, 33), (24,), 1),   # narrow planes
-    ((4, 64, 64), (30,), 0), ((4, 64, 64), (31,), 1), ((4, 64, 128), (23, 60), 1),
+    ((4, 64, 16), (15,), 0), ((4, 64, 33), (24,), 0), ((4, 64, 64), (31,), 0), ((4, 64, 128), (23, 60), 1),  # narrow planes
     ((2, 300, 300), (27,), 0), ((2, 300, 300), (3, 31), 0), ((2, 300, 300), (34,), 0), ((2, 300, 300), (35,), 1),  # few blocks
-    ((600, 256, 256), (27,), 0), ((600, 256, 256), (28,), 1), ((600, 256, 258), (31,), 0), ((600, 256, 258), (32,), 1),
-    ((900, 160, 160), (34,), 0), ((300, 256, 256), (3, 31), 0), ((300, 256, 256), (3, 32), 1),
-    ((300, 100, 128), (3, 5, 17, 32), 0), ((300, 100, 256), (3, 5, 17, 40), 1), ((60, 100, 1000), (3, 5, 17, 46), 1),
+    ((600, 256, 256), (31,), 0), ((300, 256, 256), (3, 33), 0), ((300, 256, 256), (3, 34), 1), ((300, 256, 258), (35,), 1),
+    ((300, 100, 256), (3, 5, 51), 0), ((300, 100, 256), (3, 5, 52), 1), ((60, 100, 1000), (3, 5, 17, 50), 0),
+    ((60, 100, 1000), (3, 5, 17, 51), 1), ((600, 64, 36), (17, 31), 0),
 ])
 def test_box_layer_both_ways(cuda, shape, radii, scratch):
     """Means and gradient on both sides of the choice between one launch and the way through the SAT: plane widths,
