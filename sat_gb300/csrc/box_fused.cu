@@ -332,8 +332,13 @@ __global__ void __launch_bounds__(NR * 32) box_means_kernel(const __grid_constan
 // latency at 8.4 warps an SM (the rings leave room for three blocks; issue slots 41 % busy).
 constexpr int kDGrad = 2;
 
+// Blocks an SM, for the compiler's sake: the sums turned round cost four radii off 16-byte boundaries 5 %, half of it with the
+// limit of 128 registers spoken out (us: 8 x 3 x 701 x 901, radii 5, 11, 21, 31 255 and 247).  Fewer radii and more registers go with no
+// limit given or lose (150 registers: 4096 x 32^2, radii 1, 2 63 and 69, though 64 x 3 x 1024^2 of three radii 1014 and 983).
+constexpr int grad_blocks(int nr) { return nr == 4 ? 4 : 0; }
+
 template <int NR, bool VEC>
-__global__ void __launch_bounds__(NR * 32) box_grad_kernel(const __grid_constant__ BoxArgs a, Shape sh) {
+__global__ void __launch_bounds__(NR * 32, grad_blocks(NR)) box_grad_kernel(const __grid_constant__ BoxArgs a, Shape sh) {
   constexpr int D = kDGrad;
   constexpr int T = (D * kG + NR - 1) / NR; // most outputs of a warp in a batch
   extern __shared__ __align__(16) float smem[];
