@@ -657,7 +657,7 @@ satgb_status scan_rows_strips(int in_t, int out_t, const void* d_in, int64_t in_
                               int64_t out_pitch, int64_t out_plane, int64_t width, int64_t height, int64_t planes,
                               cudaStream_t s);
 bool scan_cols_by_strips(const void* in, int64_t in_pitch, size_t in_sz, const void* out, int64_t out_pitch,
-                         size_t out_sz, int64_t width, int64_t height, int sms);
+                         size_t out_sz, int64_t width, int64_t height, bool f32, int sms);
 satgb_status scan_cols_strips(int in_t, int out_t, const void* d_in, int64_t in_pitch, void* d_out, int64_t out_pitch,
                               int64_t width, int64_t height, cudaStream_t s);
 }  // namespace satgb
@@ -736,7 +736,8 @@ satgb_status sat_single(int in_t, int out_t, int mode, int dir, const void* d_in
   if (st != SATGB_OK) return st;
   // ... nor has the column-only scan of wide images (scan_cols.cu)
   if (mode == kModeCols && dir == SATGB_FORWARD && planes == 1 &&
-      (scan_cols_by_strips(d_in, in_pitch, in_sz, d_out, out_pitch, out_sz, width, height, sms_of(dev)) ||
+      (scan_cols_by_strips(d_in, in_pitch, in_sz, d_out, out_pitch, out_sz, width, height,
+                           in_t == SATGB_F32 && out_t == SATGB_F32, sms_of(dev)) ||
        !ws_at_hand(find_variant(in_t, out_t, mode, dir, 1), width, height, 1, dev, s)))
     return scan_cols_strips(in_t, out_t, d_in, in_pitch, d_out, out_pitch, width, height, s);
   const bool off16 = planes == 1 && in_pitch == width && (uintptr_t)d_in % 16 == 0 && ((size_t)in_pitch * in_sz) % 16 != 0;

@@ -162,8 +162,11 @@ struct ColsLine {
   double start, wave, block;    // us: strips, a wave of them, a block of rows
 };
 
+// f32 sums of f32 rows on 16-byte boundaries also take strips where the older of those lines had them (3 us and 1.4 a block and wave
+// against 8 us and 5.3 TB/s): strips' two-sum pairs halve the error, and a result gets no worse.  That costs up to a fifth at
+// widths past the last wave's (10500 x 2000 40 us by tiles, 48 by strips; 6500 x 2000 26.5 and 26.9).
 bool scan_cols_by_strips(const void* in, int64_t in_pitch, size_t in_sz, const void* out, int64_t out_pitch,
-                         size_t out_sz, int64_t width, int64_t height, int sms) {
+                         size_t out_sz, int64_t width, int64_t height, bool f32, int sms) {
   const int64_t strips = (width + 31) / 32;
   if (strips >= (1LL << 31) || sms < 1) return false;
   const bool tma = (uintptr_t)in % 16 == 0 && (uintptr_t)out % 16 == 0 && ((size_t)in_pitch * in_sz) % 16 == 0 &&
@@ -171,7 +174,7 @@ bool scan_cols_by_strips(const void* in, int64_t in_pitch, size_t in_sz, const v
   const bool lines = (uintptr_t)out % 128 == 0 && ((size_t)out_pitch * out_sz) % 128 == 0;
   ColsLine c;
   if (out_sz == 4 && in_sz == 1) c = {tma ? 10.8 : 13.0, tma ? 4.8 : 2.9, 0.4, 1.1, lines ? 1.42 : 1.52};
-  else if (out_sz == 4) c = {tma ? 10.0 : 11.0, tma ? 6.0 : 3.0, 0.6, 1.1, lines ? 1.2 : 1.28};
+  else if (out_sz == 4) c = {tma ? 10.0 : 11.0, tma ? 6.0 : 3.0, 0.6, 1.1, lines ? 1.25 : 1.3};
   else if (in_sz == 1) c = {tma ? 11.9 : 12.4, tma ? 0.61 : 0.60, 1.1, 1.1, 8.9};
   else if (in_sz == 4) c = {tma ? 11.7 : 12.4, tma ? 0.81 : 0.64, 1.1, 1.1, 8.9};
   else c = {tma ? 10.2 : 10.9, tma ? 1.52 : 1.16, 1.0, 1.1, 6.9};
@@ -179,7 +182,8 @@ bool scan_cols_by_strips(const void* in, int64_t in_pitch, size_t in_sz, const v
   const double waves = (double)((strips + sms - 1) / sms);
   const double mb = (double)width * (double)height * (double)(in_sz + out_sz) * 1e-6; // a us at 1 TB/s
   const double by_strips = c.start + std::max(waves * (c.wave + blocks * c.block), mb / (lines ? 4.6 : 3.6));
-  return by_strips < c.tile_start + mb / c.tile_rate;
+  return by_strips < c.tile_start + mb / c.tile_rate ||
+         (f32 && tma && 3.0 + std::max(blocks * waves * 1.4, mb / 4.7) < 8.0 + mb / 5.3);
 }
 
 satgb_status scan_cols_strips(int in_t, int out_t, const void* d_in, int64_t in_pitch, void* d_out, int64_t out_pitch,
