@@ -8,7 +8,7 @@ the incoming gradient, one launch of the same kernel with direction=reverse.
 
 Box filter.  box_filter_means(x, radii) returns the clipped box means of every
 radius.  The plain mode takes them, and their gradient, each in one launch of
-window sums without a SAT, or through the SAT where that is faster (one call of
+window sums without a SAT, or through the SAT for large radii (one call of
 the library either way).  The compensated mode reads the four corners of the
 compensated SAT of x; its backward is the adjoint gather and the compensated reverse
 SAT in place.
