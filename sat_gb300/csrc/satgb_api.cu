@@ -1083,7 +1083,9 @@ int satgb_box_filter_fwd_x_scratch(const satgb_box_desc* desc) {
   satgb::BoxArgs a;
   if (!desc) return 0;
   satgb_box_desc d = *desc;
-  if (!d.d_sat) d.d_sat = d.d_box[0], d.sat_pitch = d.box_pitch, d.sat_plane_stride = d.box_plane_stride;
+  d.d_sat = d.d_box[0];
+  d.sat_pitch = d.box_pitch;
+  d.sat_plane_stride = d.box_plane_stride;
   if (satgb::box_check_desc(&d, a) != SATGB_OK || d.width == 0 || d.height == 0 || d.n_planes == 0) return 0;
   bool one = false;
   satgb::box_means_fused(a, nullptr, false, false, &one);

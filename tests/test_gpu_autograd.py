@@ -480,7 +480,10 @@ def test_box_layer_both_ways(cuda, shape, radii, scratch):
     w = torch.randn(shape[:1] + (len(radii),) + shape[1:], generator=g, device=cuda)
     out = torch.empty_like(w)
     import ctypes
-    assert sat_gb300._lib.load().satgb_box_filter_fwd_x_scratch(ctypes.byref(api._box_desc(x, out, radii))) == scratch
+    d = api._box_desc(x, out, radii)
+    for d_sat, pitch in ((d.d_sat, d.sat_pitch), (None, 0), (1, 0)):  # neither is looked at
+        d.d_sat, d.sat_pitch, d.sat_plane_stride = d_sat, pitch, 0
+        assert sat_gb300._lib.load().satgb_box_filter_fwd_x_scratch(ctypes.byref(d)) == scratch
     api.box_means(x, radii, out=out)
     dx = api.box_means_grad_x(w, radii)
     H, W = shape[-2:]
