@@ -33,7 +33,7 @@ const TileConfig kConfigs[kNumConfigs] = {
     {8, 8, "pipelined: 64-row tiles (32 for 8-byte accumulators), 8 warps, 2 CTAs per SM"},
     {8, 16, "registers: 128-row tiles, 16 warps"},
     {16, 16, "pipelined, 256-row tiles, direct stores (1-byte inputs, 4-byte sums)"},
-    {8, 16, "warp-specialized, direct stores: 128-row tiles (96 for 4-byte inputs, 64 for 8-byte accumulators)"},
+    {8, 16, "warp-specialized, direct stores: 128-row tiles (96 for most 4-byte inputs, 64 for 8-byte accumulators)"},
     {8, 16, "warp-specialized, direct stores, row-major tile order: 128-row tiles (64 for 8-byte accumulators)"},
 };
 
@@ -1392,8 +1392,8 @@ satgb_status plan_stage_inputs(satgb_batch_plan_s* p, const Variant* const (&vs)
   size_t total = 0;
   long long rows = 0;
   if (p->stage || p->jobs) {
-    const cudaError_t e = cudaStreamSynchronize(s); // earlier launches may still read them
-    if (e != cudaSuccess) return cuda_fail(e, "cudaStreamSynchronize");
+    const cudaError_t e = cudaDeviceSynchronize(); // earlier executions, on any stream, may still read them
+    if (e != cudaSuccess) return cuda_fail(e, "cudaDeviceSynchronize");
     ws_free(p->stage);
     if (p->jobs) cudaFree(p->jobs);
     p->stage = nullptr;
